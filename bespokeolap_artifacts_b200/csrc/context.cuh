@@ -44,6 +44,7 @@ struct bo_ctx {
   cudaStream_t copy_stream = nullptr;
   std::vector<cudaEvent_t> events;
   int stream_set = 0;  // buffer set of the streamed join's next query
+  bool join_bits_dirty = false;  // the direct join's bit table may hold bits of a call that failed half way
   // Host threads that gather the payload of matching probe rows in the
   // streamed join (-1: chosen from the machine; 0: payload read in place).
   int gather_threads = -1;
