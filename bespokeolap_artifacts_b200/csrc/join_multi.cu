@@ -9,22 +9,35 @@
 //
 // The queries are sorted by date_lt, so the queries a build row qualifies for
 // are "its segment's queries" AND "the queries with date_lt > date" -- a
-// suffix of the sorted order.  With j = the number of date_lt <= date:
-//   mask(row) = segmask[segment] & (~0u << j)
-//   count   one pass: histogram of (segment, j) per block; the last block turns
-//           it into each query's qualifying-row count and the union count
-//           (rows with a non-empty mask), which sizes the table on the device;
-//   init    clears the table for the union and the Bloom filter;
-//   build   one pass: rows with a non-empty mask insert (key << 32 | mask) with
-//           a 64-bit CAS; a key that is already present (two build rows with
-//           one key) cannot carry per-query multiplicities in one word, so it
-//           marks the whole call for an exact solo rerun of every query;
-//   probe   one pass: Bloom filter in shared memory (TMA bulk copy), the warp
-//           queue of candidates, table lookups, then per candidate the mask of
-//           queries it joins for; per round, for every query present in the
-//           warp, the warp reduces (count, T, rr) with redux.sync and lane k
-//           keeps query k's 64-bit totals; blocks add them into 128-bit totals
-//           and the last block writes every query's result.
+// suffix of its segment's queries, named by the first of them: with j = the
+// number of date_lt <= date,
+//   class(row) = first query k >= j of the row's segment (none: no query)
+// and query k's rows are those of the classes <= k of its segment.  At most 32
+// classes exist, so a key carries one byte and a matching probe row adds to one
+// class; the queries' totals are sums over classes at the end.
+//   count   one pass: rows per class, and the smallest and largest key; the last
+//           block turns them into each query's qualifying-row count and the union
+//           count (rows of any class), and decides how keys are stored:
+//   dense   one byte per key value between the smallest and the largest key,
+//           where that fits the table's memory (sixteen bytes per build row):
+//           15M dense keys are 15 MB that stay in L2;
+//   hash    else slots of key << 32 | class, sized by the union count, behind a
+//           Bloom filter;
+//   init    clears whichever it is;
+//   build   one pass: rows with a class store it; a key that is already present
+//           (two build rows with one key) cannot carry per-query multiplicities
+//           in one byte, so it marks the whole call for an exact solo rerun of
+//           every query;
+//   probe   one pass: each matching row adds its count, T and rr to its class in
+//           the warp's shared-memory accumulators; blocks add the classes' totals
+//           into 128-bit totals and the last block writes every query's result.
+// The kernels of the form that was not chosen return at once.  Measured (B200,
+// build 15M, probe 60M, 16 queries, dense keys): 478 us a call (count 62, build
+// 108, probe 305) against 2934 us with a query mask per hashed slot and a warp
+// reduction per query; keys over the whole 32-bit range (hash): 2703 against
+// 2950 us, 25K x 100K rows: 41 and 66 against 77 us.  The line between the forms
+// is the table's memory and no lower: just inside it (keys ten apart) dense
+// takes 885 us for 2 queries, hash 1656 us just outside (twenty apart).
 #include <algorithm>
 #include <numeric>
 
@@ -39,11 +52,11 @@ constexpr int kMq = BO_JOIN_MULTI_MAX;  // queries per call (one mask bit each)
 constexpr int kMqBlock = 512;
 constexpr int kMqBuildBlock = 256;
 constexpr int kMqRowsPerLane = 8;       // probe rows per lane per warp step
-constexpr int kMqBuildRows = 16;        // build rows per thread
+constexpr int kMqBuildRows = 8;         // build rows per thread
 constexpr int kMqWarps = kMqBlock / 32;
 constexpr int kMqMinCapLog2 = 10;
 
-// Predicate constants, queries in date_lt order (sorted index k = mask bit k).
+// Predicate constants, queries in date_lt order (sorted index k).
 struct MultiQ {
   int32_t n;
   int32_t n_seg;                 // distinct segments among the queries
@@ -55,16 +68,25 @@ struct MultiQ {
 };
 
 // Device state of one call ("join_multi_meta" region; cleared by the host
-// before every call).
+// before every call).  Class codes are 1 + the class's first query; 0 is none.
 struct MqState {
-  unsigned long long hist[kMq * (kMq + 1)];  // [compact segment][j]
+  unsigned long long hist[kMq + 1];          // rows per class code
   unsigned long long count[kMq];             // qualifying rows per sorted query
-  unsigned long long acc[kMq * 6];           // per query 128-bit match count, sum T, sum rr
+  unsigned long long acc[kMq * 6];           // per class 128-bit match count, sum T, sum rr
   unsigned long long distinct;
+  uint32_t key_max, key_nmin;                // largest key and largest ~key, in unsigned order
+  uint32_t base, range;                      // dense: smallest key, key values from it to the largest
   uint32_t ticket_count, ticket_probe, dup, overflow;
-  int32_t cap_log2;
+  int32_t cap_log2, dense;
   float union_rows;
 };
+
+__device__ __forceinline__ void mq_load_queries(MultiQ& q, const MultiQ& qv) {
+  static_assert(sizeof(MultiQ) % 4 == 0, "copied in words");
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(&qv);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(&q);
+  for (int i = threadIdx.x; i < (int)(sizeof(MultiQ) / 4); i += blockDim.x) dst[i] = src[i];
+}
 
 __device__ __forceinline__ uint32_t mq_first_above(const int32_t* date_lt, int n, int32_t date) {
   uint32_t lo = 0, hi = (uint32_t)n;  // first sorted query with date_lt > date
@@ -78,41 +100,98 @@ __device__ __forceinline__ uint32_t mq_first_above(const int32_t* date_lt, int n
 
 __device__ __forceinline__ uint32_t mq_suffix(uint32_t j) { return j >= 32u ? 0u : (~0u << j); }
 
-__device__ __forceinline__ uint32_t mq_mask(const MultiQ& q, int32_t date, uint32_t seg_byte) {
+// Class code of a build row (0: no query wants it).
+__device__ __forceinline__ uint32_t mq_class(const MultiQ& q, int32_t date, uint32_t seg_byte) {
   const int idx = q.seg_idx[seg_byte & 0xffu];
   if (idx < 0) return 0u;
-  return q.segmask[idx] & mq_suffix(mq_first_above(q.date_lt, q.n, date));
+  return (uint32_t)__ffs((int)(q.segmask[idx] & mq_suffix(mq_first_above(q.date_lt, q.n, date))));
+}
+
+// Class codes and keys of the kRows build rows from r0 on (codes 0 past the end).
+template <int kRows>
+__device__ __forceinline__ void mq_build_rows(const bo_join_build_cols& b, const MultiQ& q, int64_t r0,
+                                              uint32_t (&code)[kRows], uint32_t (&key)[kRows]) {
+  static_assert(kRows == 8, "one 256-bit load of dates and of keys");
+  if (r0 + kRows <= b.n_rows) {
+    const uint2 sg = ld_stream_v2(b.segment + r0);
+    const int8v d = ld_first_v8(b.date + r0), k = ld_first_v8(b.key + r0);
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      code[j] = mq_class(q, d.v[j], (j < 4 ? sg.x : sg.y) >> (8 * (j & 3)));
+      key[j] = (uint32_t)k.v[j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      code[j] = 0;
+      key[j] = 0;
+      if (r0 + j < b.n_rows) {
+        code[j] = mq_class(q, b.date[r0 + j], b.segment[r0 + j]);
+        key[j] = (uint32_t)b.key[r0 + j];
+      }
+    }
+  }
 }
 
 // --------------------------------------------------------------- count ---
-__global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_cols b, MultiQ qv, MqState* st) {
+constexpr uint32_t kSign = 0x80000000u;  // int32 order as uint32 order
+
+__global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_cols b, MultiQ qv, MqState* st,
+                                                                 uint32_t dense_max) {
+  constexpr int kCopies = 8;  // of each class's counter: lanes of one class spread over them
   __shared__ MultiQ q;
-  __shared__ uint32_t h[kMq * (kMq + 1)];
-  if (threadIdx.x == 0) q = qv;
-  for (int i = threadIdx.x; i < kMq * (kMq + 1); i += kMqBuildBlock) h[i] = 0;
+  __shared__ uint32_t h[(kMq + 1) * kCopies];
+  __shared__ unsigned long long tot[kMq + 1];
+  mq_load_queries(q, qv);
+  for (int i = threadIdx.x; i < (kMq + 1) * kCopies; i += kMqBuildBlock) h[i] = 0;
   __syncthreads();
-  const int64_t n = b.n_rows;
-  for (int64_t i = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * kMqBuildBlock) {
-    const int idx = q.seg_idx[b.segment[i]];
-    if (idx < 0) continue;
-    atomicAdd(h + idx * (kMq + 1) + mq_first_above(q.date_lt, q.n, b.date[i]), 1u);
+  const int lane = threadIdx.x & 31;
+  const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
+  uint32_t kmax = 0, nmin = 0;
+  for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
+       c += (int64_t)gridDim.x * kMqBuildBlock) {
+    uint32_t code[kMqBuildRows], key[kMqBuildRows];
+    mq_build_rows(b, q, c * kMqBuildRows, code, key);
+#pragma unroll
+    for (int j = 0; j < kMqBuildRows; ++j) {
+      if (!code[j]) continue;
+      atomicAdd(h + code[j] * kCopies + (lane & (kCopies - 1)), 1u);
+      const uint32_t k = key[j] ^ kSign;
+      kmax = max(kmax, k);
+      nmin = max(nmin, ~k);
+    }
+  }
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  nmin = __reduce_max_sync(0xffffffffu, nmin);
+  if (lane == 0 && (kmax | nmin)) {
+    atomicMax(&st->key_max, kmax);
+    atomicMax(&st->key_nmin, nmin);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < q.n_seg * (kMq + 1); i += kMqBuildBlock)
-    if (h[i]) atomicAdd(st->hist + i, (unsigned long long)h[i]);
-  if (last_block(&st->ticket_count) && threadIdx.x == 0) {
-    // query k (segment s = seg_of[k]) counts the rows of segment s with j <= k
-    for (int k = 0; k < q.n; ++k) {
-      unsigned long long c = 0;
-      for (int j = 0; j <= k; ++j) c += __ldcg(st->hist + q.seg_of[k] * (kMq + 1) + j);
-      st->count[k] = c;
-    }
+  if (threadIdx.x <= kMq) {
+    uint32_t t = 0;
+    for (int i = 0; i < kCopies; ++i) t += h[threadIdx.x * kCopies + i];
+    if (t) atomicAdd(st->hist + threadIdx.x, (unsigned long long)t);
+  }
+  if (!last_block(&st->ticket_count)) return;
+  if (threadIdx.x <= kMq) tot[threadIdx.x] = __ldcg(st->hist + threadIdx.x);
+  __syncthreads();
+  if (threadIdx.x < q.n) {
+    const uint32_t k = threadIdx.x;
+    unsigned long long c = 0;
+    for (uint32_t j = 0; j <= k; ++j)
+      if (q.seg_of[j] == q.seg_of[k]) c += tot[j + 1];
+    st->count[k] = c;
+  }
+  if (threadIdx.x == 0) {
     unsigned long long u = 0;
-    for (int s = 0; s < q.n_seg; ++s)
-      for (int j = 0; j <= q.n; ++j)
-        if (q.segmask[s] & mq_suffix((uint32_t)j)) u += __ldcg(st->hist + s * (kMq + 1) + j);
+    for (int k = 1; k <= kMq; ++k) u += tot[k];
+    const uint32_t lo = ~__ldcg(&st->key_nmin), hi = __ldcg(&st->key_max);
+    const uint64_t range = u ? (uint64_t)hi - lo + 1 : 0;
     st->union_rows = (float)u;
+    st->dense = range <= dense_max;
+    st->base = lo ^ kSign;
+    st->range = (uint32_t)range;
   }
 }
 
@@ -121,21 +200,52 @@ __global__ void mq_init_kernel(unsigned long long* slots, uint32_t* bloom, MqSta
   const double want = (double)st->union_rows * 2.0;  // exact count: load <= 0.5
   int32_t cl = kMqMinCapLog2;
   while (cl < max_log2 && (double)(1ull << cl) < want) ++cl;
-  const uint64_t cap = 1ull << cl;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid == 0) st->cap_log2 = cl;
+  if (st->dense) {
+    uint4* v = reinterpret_cast<uint4*>(slots);
+    for (uint64_t i = tid; i < ((uint64_t)st->range + 15) / 16; i += stride) v[i] = make_uint4(0, 0, 0, 0);
+    return;
+  }
+  const uint64_t cap = 1ull << cl;
   ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
   for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
   uint4* b4 = reinterpret_cast<uint4*>(bloom);
   for (uint64_t i = tid; i < kBloomWords / 4; i += stride) b4[i] = make_uint4(0, 0, 0, 0);
-  if (tid == 0) st->cap_log2 = cl;
 }
 
 // --------------------------------------------------------------- build ---
+// Dense: the class byte is ORed into its word, the old byte tells a repeated
+// key; a thread's atomics are all issued before any old value is used.
+__global__ void __launch_bounds__(kMqBuildBlock) mq_build_dense_kernel(bo_join_build_cols b, MultiQ qv,
+                                                                       uint32_t* __restrict__ bytes, MqState* st) {
+  if (!__ldg(&st->dense)) return;
+  __shared__ MultiQ q;
+  mq_load_queries(q, qv);
+  __syncthreads();
+  const uint32_t base = __ldg(&st->base);
+  const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
+  uint32_t dup = 0;
+  for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
+       c += (int64_t)gridDim.x * kMqBuildBlock) {
+    uint32_t code[kMqBuildRows], key[kMqBuildRows], old[kMqBuildRows];
+    mq_build_rows(b, q, c * kMqBuildRows, code, key);
+#pragma unroll
+    for (int j = 0; j < kMqBuildRows; ++j) {
+      const uint32_t off = key[j] - base;
+      old[j] = code[j] ? atomicOr(bytes + (off >> 2), code[j] << (8 * (off & 3u))) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kMqBuildRows; ++j) dup |= (old[j] >> (8 * ((key[j] - base) & 3u))) & 0xffu;
+  }
+  if (__any_sync(0xffffffffu, dup != 0) && (threadIdx.x & 31) == 0) atomicOr(&st->dup, 1u);
+}
+
 __device__ __forceinline__ void mq_insert(unsigned long long* slots, uint32_t* bloom, uint64_t mask, int32_t key,
-                                          uint32_t qmask, uint32_t& newkeys, uint32_t& dup, uint32_t& full) {
+                                          uint32_t code, uint32_t& newkeys, uint32_t& dup, uint32_t& full) {
   uint64_t idx = hash32((uint32_t)key) & mask;
-  const unsigned long long mine = ((unsigned long long)(uint32_t)key << 32) | qmask;
+  const unsigned long long mine = ((unsigned long long)(uint32_t)key << 32) | code;
   for (uint64_t step = 0; step <= mask; ++step) {
     const unsigned long long old = atomicCAS(slots + idx, kEmptySlot, mine);
     if (old == kEmptySlot) {
@@ -157,55 +267,33 @@ __device__ __forceinline__ void mq_insert(unsigned long long* slots, uint32_t* b
 __global__ void __launch_bounds__(kMqBuildBlock) mq_build_kernel(bo_join_build_cols b, MultiQ qv,
                                                                  unsigned long long* slots, uint32_t* bloom,
                                                                  MqState* st) {
+  if (__ldg(&st->dense)) return;
   __shared__ MultiQ q;
   __shared__ uint32_t queue[kMqBuildBlock / 32][2][32 * kMqBuildRows];
-  if (threadIdx.x == 0) q = qv;
+  mq_load_queries(q, qv);
   __syncthreads();
   const uint64_t mask = (1ull << __ldcg(&st->cap_log2)) - 1;
   const int lane = threadIdx.x & 31;
   uint32_t* qk = queue[threadIdx.x >> 5][0];
   uint32_t* qm = queue[threadIdx.x >> 5][1];
   uint32_t newkeys = 0, dup = 0, full = 0;
-  const int64_t n = b.n_rows;
-  const int64_t steps = (n + kMqBuildRows - 1) / kMqBuildRows;
+  const int64_t steps = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
   const int64_t steps_w = (steps + 31) & ~int64_t(31);  // whole warps: the queue steps stay converged
   for (int64_t s = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; s < steps_w;
        s += (int64_t)gridDim.x * kMqBuildBlock) {
-    const int64_t r0 = s * kMqBuildRows;
-    int32_t keys[kMqBuildRows];
-    uint32_t qms[kMqBuildRows];
+    uint32_t code[kMqBuildRows], key[kMqBuildRows];
+    mq_build_rows(b, q, s * kMqBuildRows, code, key);
     uint32_t any = 0;
-    if (r0 + kMqBuildRows <= n) {
-      const int4 sg = ld_stream_v4(b.segment + r0);
-      const uint32_t sw[4] = {(uint32_t)sg.x, (uint32_t)sg.y, (uint32_t)sg.z, (uint32_t)sg.w};
-      const int8v d0 = ld_stream_v8(b.date + r0), d1 = ld_stream_v8(b.date + r0 + 8);
-      const int8v k0 = ld_stream_v8(b.key + r0), k1 = ld_stream_v8(b.key + r0 + 8);
 #pragma unroll
-      for (int k = 0; k < kMqBuildRows; ++k) {
-        qms[k] = mq_mask(q, k < 8 ? d0.v[k] : d1.v[k - 8], sw[k >> 2] >> (8 * (k & 3)));
-        keys[k] = k < 8 ? k0.v[k] : k1.v[k - 8];
-        any |= (qms[k] != 0u) << k;
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < kMqBuildRows; ++k) {
-        qms[k] = 0;
-        keys[k] = 0;
-        if (r0 + k < n) {
-          qms[k] = mq_mask(q, b.date[r0 + k], b.segment[r0 + k]);
-          keys[k] = b.key[r0 + k];
-          any |= (qms[k] != 0u) << k;
-        }
-      }
-    }
+    for (int k = 0; k < kMqBuildRows; ++k) any |= (uint32_t)(code[k] != 0u) << k;
     uint32_t total;
     uint32_t pos = warp_exclusive_scan(__popc(any), total);
     if (total == 0) continue;  // warp-uniform
 #pragma unroll
     for (int k = 0; k < kMqBuildRows; ++k)
       if ((any >> k) & 1u) {
-        qk[pos] = (uint32_t)keys[k];
-        qm[pos] = qms[k];
+        qk[pos] = key[k];
+        qm[pos] = code[k];
         ++pos;
       }
     __syncwarp();
@@ -222,18 +310,151 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_build_kernel(bo_join_build_c
 }
 
 // --------------------------------------------------------------- probe ---
-// Per-lane totals of the query this lane owns (lane k <-> sorted query k).
+// Per-class sums of one warp in shared memory, 32-bit words added to by
+// atomics; four copies of each class (by lane) keep lanes of one class from
+// queueing on one word.  A matching row adds T in two 16-bit halves and
+// 1 << 20 | rr (rr < 100): at most kMqFlush rows may be added before a flush.
+constexpr int kMqCopies = 4;
+constexpr int kMqAccWords = 3;
+constexpr uint32_t kMqFlush = 4095;  // count < 2^12 above bit 20; sum rr < 2^19; halves < 2^28
+
+struct MqWarpAcc {
+  uint32_t w[kMqAccWords][kMq * kMqCopies];
+};
+
+// Lane k's 64-bit totals of class k, taken out of the warp's accumulators.
 struct MqAcc {
   unsigned long long cnt = 0, t = 0, rr = 0;
   uint32_t bad = 0;
 };
 
+__device__ __forceinline__ void mq_flush(MqWarpAcc& wa, MqAcc& acc) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < kMqCopies; ++c) {
+    const int i = lane * kMqCopies + c;
+    const uint32_t lo = wa.w[0][i], hi = wa.w[1][i], pk = wa.w[2][i];
+    wa.w[0][i] = wa.w[1][i] = wa.w[2][i] = 0;
+    acc.cnt += pk >> 20;
+    acc.rr += pk & 0xfffffu;
+    acc.t += lo + ((unsigned long long)hi << 16);
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ void mq_add(MqWarpAcc& wa, uint32_t code, uint64_t p, uint64_t d, MqAcc& acc) {
+  if (p >= 0x80000000ull || d > 100u) {
+    acc.bad |= kErrValueRange;
+    return;
+  }
+  const uint32_t m = 100u - (uint32_t)d, pq = (uint32_t)p / 100u, pr = (uint32_t)p - pq * 100u;
+  const uint32_t rm = pr * m, rq = rm / 100u, T = pq * m + rq;
+  const uint32_t i = (code - 1u) * kMqCopies + (threadIdx.x & (kMqCopies - 1));
+  atomicAdd(&wa.w[0][i], T & 0xffffu);
+  atomicAdd(&wa.w[1][i], T >> 16);
+  atomicAdd(&wa.w[2][i], (1u << 20) | (rm - rq * 100u));
+}
+
+// The block's totals per class into the 128-bit totals; the last block writes
+// every query's result (the sum of its segment's classes up to it).
+__device__ __forceinline__ void mq_finish(MqWarpAcc* wa, int warps, MqAcc& acc, MqState* st, const MultiQ& qv,
+                                          bo_join_result* out, uint32_t* err) {
+  __shared__ __int128 cls[kMq][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  mq_flush(wa[warp], acc);
+  if (acc.bad) raise_error(err, acc.bad);
+  // The accumulators' memory now carries each warp's 64-bit totals.
+  static_assert(sizeof(MqWarpAcc) >= sizeof(unsigned long long) * 3 * 32, "per-warp totals fit");
+  unsigned long long* mine = reinterpret_cast<unsigned long long*>(wa + warp);
+  mine[lane * 3] = acc.cnt;
+  mine[lane * 3 + 1] = acc.t;
+  mine[lane * 3 + 2] = acc.rr;
+  __syncthreads();
+  if (threadIdx.x < 32 * 3) {
+    unsigned long long v = 0;  // per block: < 2^32 rows x < 2^31, fits 64 bits
+    for (int w = 0; w < warps; ++w) v += reinterpret_cast<unsigned long long*>(wa + w)[threadIdx.x];
+    if (v) atomic_add_i128(st->acc + 2 * threadIdx.x, (__int128)v);
+  }
+  if (!last_block(&st->ticket_probe)) return;
+  if (threadIdx.x < 32 * 3) cls[threadIdx.x / 3][threadIdx.x % 3] = load_i128(st->acc + 2 * threadIdx.x);
+  __syncthreads();
+  if (threadIdx.x < qv.n) {
+    const int k = threadIdx.x;
+    uint32_t fbad = 0;
+    __int128 m = 0, t = 0, rr = 0;
+    for (int c = 0; c <= k; ++c)
+      if (qv.seg_of[c] == qv.seg_of[k]) {
+        m += cls[c][0];
+        t += cls[c][1];
+        rr += cls[c][2];
+      }
+    bo_join_result r;
+    r.build_rows = (int64_t)__ldcg(&st->count[k]);
+    r.distinct_keys = r.build_rows;  // no key repeats (else the call is marked for rerun)
+    r.match_count = narrow_i64(m, fbad);
+    r.sum_trunc = to_bo_i128(t);
+    r.sum_exact = to_bo_i128(t * 100 + rr);
+    r.capacity_log2 = __ldcg(&st->cap_log2);
+    r.overflowed = (int32_t)(__ldcg(&st->dup) | __ldcg(&st->overflow));
+    r.reruns = 0;
+    r.mode = 0;
+    out[qv.perm[k]] = r;
+    if (fbad) raise_error(err, fbad);
+  }
+}
+
+// Dense: a warp owns 256 consecutive rows per step, lane-strided (row base + 32 j
+// + lane) so that the price / discount loads of one j coalesce.  Bound by the
+// random byte loads: L1 79% and L2 71% busy, DRAM 48% (305 us for 60M rows).
+constexpr int kMqDenseBlock = 256;
+
+__global__ void __launch_bounds__(kMqDenseBlock) mq_probe_dense_kernel(bo_join_probe_cols p,
+                                                                       const uint8_t* __restrict__ bytes, MqState* st,
+                                                                       bo_join_result* out, MultiQ qv, uint32_t* err) {
+  if (!__ldg(&st->dense)) return;
+  constexpr int kWarps = kMqDenseBlock / 32;
+  __shared__ __align__(16) MqWarpAcc wa[kWarps];
+  for (int i = threadIdx.x; i < (int)(sizeof(wa) / 4); i += kMqDenseBlock) reinterpret_cast<uint32_t*>(wa)[i] = 0;
+  __syncthreads();
+  const uint32_t base_key = __ldg(&st->base), range = __ldg(&st->range);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = p.n_rows;
+  constexpr int kStep = 32 * kMqRowsPerLane;
+  const int64_t steps = (n + kStep - 1) / kStep;
+  MqAcc acc;
+  uint32_t added = 0;
+  for (int64_t s = (int64_t)blockIdx.x * kWarps + warp; s < steps; s += (int64_t)gridDim.x * kWarps) {
+    const int64_t r0 = s * kStep + lane;
+    uint32_t off[kMqRowsPerLane], code[kMqRowsPerLane];
+#pragma unroll
+    for (int j = 0; j < kMqRowsPerLane; ++j)
+      off[j] = r0 + 32 * j < n ? (uint32_t)__ldcs(p.fk + r0 + 32 * j) - base_key : ~0u;
+#pragma unroll
+    for (int j = 0; j < kMqRowsPerLane; ++j) code[j] = off[j] < range ? __ldg(bytes + off[j]) : 0u;
+    uint64_t pr[kMqRowsPerLane], dc[kMqRowsPerLane];
+#pragma unroll
+    for (int j = 0; j < kMqRowsPerLane; ++j) {
+      pr[j] = code[j] ? (uint64_t)__ldcs(p.price + r0 + 32 * j) : 0u;
+      dc[j] = code[j] ? (uint64_t)__ldcs(p.discount + r0 + 32 * j) : 0u;
+    }
+    if (added + kStep > kMqFlush) {
+      mq_flush(wa[warp], acc);
+      added = 0;
+    }
+    added += kStep;
+#pragma unroll
+    for (int j = 0; j < kMqRowsPerLane; ++j)
+      if (code[j]) mq_add(wa[warp], code[j], pr[j], dc[j], acc);
+  }
+  mq_finish(wa, kWarps, acc, st, qv, out, err);
+}
+
 // Resolves the warp's queued candidates (as probe_resolve in rows.cuh, R = 2
-// per lane per round), then reduces each present query's (count, T, rr) over
-// the warp; T is split in 16-bit halves so every warp sum fits 32 bits.
-__device__ __forceinline__ void mq_resolve(const int32_t* qf, const uint16_t* qo, uint32_t total, int64_t base,
+// per lane per round) and adds the matches to their classes.
+__device__ __forceinline__ void mq_resolve(const int32_t* qf, const uint8_t* qo, uint32_t total, int64_t base,
                                            const unsigned long long* slots, uint64_t mask, const int64_t* price,
-                                           const int64_t* disc, MqAcc& acc) {
+                                           const int64_t* disc, MqWarpAcc& wa, MqAcc& acc) {
   constexpr int R = 2;
   const int lane = threadIdx.x & 31;
   for (uint32_t i0 = 0; i0 < total; i0 += 32 * R) {
@@ -250,69 +471,40 @@ __device__ __forceinline__ void mq_resolve(const int32_t* qf, const uint16_t* qo
       idx[r] = hash32((uint32_t)key[r]) & mask;
       v[r] = ok ? __ldg(slots + idx[r]) : kEmptySlot;
     }
-    uint32_t m[R];
+    uint32_t code[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      m[r] = 0;
+      code[r] = 0;
       if (v[r] != kEmptySlot) {
         if ((uint32_t)(v[r] >> 32) == (uint32_t)key[r])
-          m[r] = (uint32_t)v[r];
+          code[r] = (uint32_t)v[r];
         else
-          m[r] = (uint32_t)probe_slow<false>(slots, mask, idx[r], (uint32_t)key[r], ~0ull);
+          code[r] = (uint32_t)probe_slow<false>(slots, mask, idx[r], (uint32_t)key[r], ~0ull);
       }
     }
-    uint32_t T[R], rr[R];
+    uint64_t pr[R], dc[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      T[r] = 0;
-      rr[r] = 0;
-      if (m[r]) {
-        const uint64_t p = (uint64_t)__ldg(price + row[r]), d = (uint64_t)__ldg(disc + row[r]);
-        if (p >= 0x80000000ull || d > 100u) {
-          acc.bad |= kErrValueRange;
-          m[r] = 0;
-          continue;
-        }
-        const uint32_t mm = 100u - (uint32_t)d, pq = (uint32_t)p / 100u, pr = (uint32_t)p - pq * 100u;
-        const uint32_t rm = pr * mm, rq = rm / 100u;
-        T[r] = pq * mm + rq;
-        rr[r] = rm - rq * 100u;
-      }
+      pr[r] = code[r] ? (uint64_t)__ldg(price + row[r]) : 0u;
+      dc[r] = code[r] ? (uint64_t)__ldg(disc + row[r]) : 0u;
     }
-    uint32_t present = __reduce_or_sync(0xffffffffu, m[0] | m[1]);
-    while (present) {
-      const int k = __ffs(present) - 1;
-      present &= present - 1;
-      uint32_t c = 0, tl = 0, th = 0, rs = 0;
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        if ((m[r] >> k) & 1u) {
-          ++c;
-          tl += T[r] & 0xffffu;
-          th += T[r] >> 16;
-          rs += rr[r];
-        }
-      c = __reduce_add_sync(0xffffffffu, c);
-      tl = __reduce_add_sync(0xffffffffu, tl);
-      th = __reduce_add_sync(0xffffffffu, th);
-      rs = __reduce_add_sync(0xffffffffu, rs);
-      if (lane == k) {
-        acc.cnt += c;
-        acc.t += (unsigned long long)tl + ((unsigned long long)th << 16);
-        acc.rr += rs;
-      }
-    }
+    for (int r = 0; r < R; ++r)
+      if (code[r]) mq_add(wa, code[r], pr[r], dc[r], acc);
   }
 }
 
 __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_cols p, const unsigned long long* slots,
                                                               const uint32_t* bloom_g, MqState* st,
                                                               bo_join_result* out, MultiQ qv, uint32_t* err) {
+  if (__ldg(&st->dense)) return;
   extern __shared__ __align__(128) uint32_t bloom_s[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int32_t q_fk[kMqWarps][32 * kMqRowsPerLane];
-  __shared__ uint16_t q_off[kMqWarps][32 * kMqRowsPerLane];
-  __shared__ unsigned long long part[kMqWarps][32][3];
+  __shared__ uint8_t q_off[kMqWarps][32 * kMqRowsPerLane];
+  MqWarpAcc* wa = reinterpret_cast<MqWarpAcc*>(bloom_s + kBloomWords);
+  for (int i = threadIdx.x; i < (int)(kMqWarps * sizeof(MqWarpAcc) / 4); i += kMqBlock)
+    reinterpret_cast<uint32_t*>(wa)[i] = 0;
   if (threadIdx.x == 0) {
     mbar_init(&bar, 1);
     mbar_arrive_expect_tx(&bar, kBloomBytes);
@@ -331,10 +523,11 @@ __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_col
   const uint64_t mask = (1ull << __ldcg(&st->cap_log2)) - 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int32_t* qf = q_fk[warp];
-  uint16_t* qo = q_off[warp];
+  uint8_t* qo = q_off[warp];
   const int64_t n = p.n_rows;
   constexpr int kStep = 32 * kMqRowsPerLane;
   const int64_t steps = (n + kStep - 1) / kStep;
+  uint32_t added = 0;
   for (int64_t s = (int64_t)blockIdx.x * kMqWarps + warp; s < steps; s += (int64_t)gridDim.x * kMqWarps) {
     const int64_t base = s * kStep;
     const int64_t r0 = base + lane * kMqRowsPerLane;
@@ -365,43 +558,20 @@ __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_col
     for (int k = 0; k < kMqRowsPerLane; ++k)
       if ((hit >> k) & 1u) {
         qf[pos] = fk[k];
-        qo[pos] = (uint16_t)(lane * kMqRowsPerLane + k);
+        qo[pos] = (uint8_t)(lane * kMqRowsPerLane + k);
         ++pos;
       }
+    if (added + total > kMqFlush) {
+      mq_flush(wa[warp], acc);
+      added = 0;
+    }
+    added += total;
     __syncwarp();
-    mq_resolve(qf, qo, total, base, slots, mask, p.price, p.discount, acc);
+    mq_resolve(qf, qo, total, base, slots, mask, p.price, p.discount, wa[warp], acc);
     __syncwarp();
   }
   if (!use_bloom) mbar_wait_bounded(&bar, 0, kWaitLimitNs);  // the copy may still be in flight
-  if (acc.bad) raise_error(err, acc.bad);
-  part[warp][lane][0] = acc.cnt;
-  part[warp][lane][1] = acc.t;
-  part[warp][lane][2] = acc.rr;
-  __syncthreads();
-  if (threadIdx.x < 32 * 3) {
-    const int k = threadIdx.x / 3, f = threadIdx.x % 3;
-    unsigned long long v = 0;  // per block: < 2^32 rows x < 2^31, fits 64 bits
-    for (int w = 0; w < kMqWarps; ++w) v += part[w][k][f];
-    if (v) atomic_add_i128(st->acc + 6 * k + 2 * f, (__int128)v);
-  }
-  if (last_block(&st->ticket_probe) && threadIdx.x < qv.n) {
-    const int k = threadIdx.x;
-    uint32_t fbad = 0;
-    const __int128 m = load_i128(st->acc + 6 * k), t = load_i128(st->acc + 6 * k + 2),
-                   rr = load_i128(st->acc + 6 * k + 4);
-    bo_join_result r;
-    r.build_rows = (int64_t)__ldcg(&st->count[k]);
-    r.distinct_keys = r.build_rows;  // no key repeats (else the call is marked for rerun)
-    r.match_count = narrow_i64(m, fbad);
-    r.sum_trunc = to_bo_i128(t);
-    r.sum_exact = to_bo_i128(t * 100 + rr);
-    r.capacity_log2 = __ldcg(&st->cap_log2);
-    r.overflowed = (int32_t)(__ldcg(&st->dup) | __ldcg(&st->overflow));
-    r.reruns = 0;
-    r.mode = 0;
-    out[qv.perm[k]] = r;
-    if (fbad) raise_error(err, fbad);
-  }
+  mq_finish(wa, kMqWarps, acc, st, qv, out, err);
 }
 
 int ceil_log2_u64(uint64_t v) {
@@ -470,25 +640,37 @@ extern "C" int bo_join_multi_device(bo_ctx* ctx, const bo_join_build_cols* b, co
   auto* st = static_cast<MqState*>(ptr);
   BO_CUDA(ctx, cudaMemsetAsync(st, 0, sizeof(MqState), ctx->stream));
 
+  // Dense form while the key values from smallest to largest fit the table's memory.
+  const uint32_t dense_max = (uint32_t)std::min<uint64_t>(sizeof(unsigned long long) << max_log2, 0xfffffff0ull);
+  const int64_t chunks = (b->n_rows + kMqBuildRows - 1) / kMqBuildRows;
   const void* kc = reinterpret_cast<const void*>(&mq_count_kernel);
-  mq_count_kernel<<<mq_grid(ctx, kc, kMqBuildBlock, 0, b->n_rows), kMqBuildBlock, 0, ctx->stream>>>(*b, q, st);
+  mq_count_kernel<<<mq_grid(ctx, kc, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(*b, q, st, dense_max);
   if ((rc = after_launch(ctx, "mq_count_kernel"))) return rc;
   const void* ki = reinterpret_cast<const void*>(&mq_init_kernel);
   mq_init_kernel<<<mq_grid(ctx, ki, 256, 0, (int64_t)1 << std::min(max_log2, 24)), 256, 0, ctx->stream>>>(
       slots, bloom, st, max_log2);
   if ((rc = after_launch(ctx, "mq_init_kernel"))) return rc;
+  const void* kd = reinterpret_cast<const void*>(&mq_build_dense_kernel);
+  mq_build_dense_kernel<<<mq_grid(ctx, kd, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(
+      *b, q, reinterpret_cast<uint32_t*>(slots), st);
+  if ((rc = after_launch(ctx, "mq_build_dense_kernel"))) return rc;
   const void* kb = reinterpret_cast<const void*>(&mq_build_kernel);
-  mq_build_kernel<<<mq_grid(ctx, kb, kMqBuildBlock, 0, (b->n_rows + kMqBuildRows - 1) / kMqBuildRows),
-                    kMqBuildBlock, 0, ctx->stream>>>(*b, q, slots, bloom, st);
+  mq_build_kernel<<<mq_grid(ctx, kb, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(*b, q, slots, bloom, st);
   if ((rc = after_launch(ctx, "mq_build_kernel"))) return rc;
+  const int64_t lanes = (p->n_rows + kMqRowsPerLane - 1) / kMqRowsPerLane;
+  const void* kq = reinterpret_cast<const void*>(&mq_probe_dense_kernel);
+  mq_probe_dense_kernel<<<mq_grid(ctx, kq, kMqDenseBlock, 0, lanes), kMqDenseBlock, 0, ctx->stream>>>(
+      *p, reinterpret_cast<const uint8_t*>(slots), st, out_device, q, ctx->d_err);
+  if ((rc = after_launch(ctx, "mq_probe_dense_kernel"))) return rc;
   const void* kp = reinterpret_cast<const void*>(&mq_probe_kernel);
+  constexpr size_t smem = kBloomBytes + kMqWarps * sizeof(MqWarpAcc);
   static bool ready = false;
   if (!ready) {
-    BO_CUDA(ctx, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBloomBytes));
+    BO_CUDA(ctx, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ready = true;
   }
-  const int gp = mq_grid(ctx, kp, kMqBlock, kBloomBytes, (p->n_rows + kMqRowsPerLane - 1) / kMqRowsPerLane);
-  mq_probe_kernel<<<gp, kMqBlock, kBloomBytes, ctx->stream>>>(*p, slots, bloom, st, out_device, q, ctx->d_err);
+  mq_probe_kernel<<<mq_grid(ctx, kp, kMqBlock, smem, lanes), kMqBlock, smem, ctx->stream>>>(*p, slots, bloom, st,
+                                                                                           out_device, q, ctx->d_err);
   return after_launch(ctx, "mq_probe_kernel");
 }
 

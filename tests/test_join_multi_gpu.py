@@ -89,3 +89,49 @@ def test_join_multi_device_async_and_limits(engine, torch_cuda):
 def C_sizeof():
     import ctypes
     return ctypes.sizeof(N.JoinResult)
+
+
+@pytest.mark.parametrize("spread", ["dense", "negative", "whole_range", "at_limit", "past_limit"])
+def test_join_multi_key_ranges(engine, torch_cuda, spread):
+    """Both table forms: one byte per key value while the range from the smallest to the largest key fits 16 bytes per
+    build row (rounded up to a power of two), hashed slots beyond it; fks outside the keys' range on both sides."""
+    nb, npr, nq = 100_000, 700_003, 32
+    j = dg.gen_join(nb, npr, seed=31)
+    rng = np.random.default_rng(32)
+    limit = 8 << 18  # table bytes for 100,000 rows: 2^18 slots of 8 bytes
+    hi = {"dense": nb, "negative": nb, "whole_range": 2**32, "at_limit": limit, "past_limit": limit + 1}[spread]
+    lo = {"dense": 1, "negative": -nb // 2, "whole_range": -2**31}.get(spread, -77)
+    key = lo + rng.choice(min(hi, 4_000_000), nb, replace=False).astype(np.int64) * max(1, hi // 4_000_000)
+    key[:2] = lo, lo + hi - 1  # the ends of the range, kept unique and always qualifying
+    _, first = np.unique(key, return_index=True)
+    key = key[np.sort(first)]
+    date, seg = j.b_date[:len(key)].copy(), j.b_seg[:len(key)].copy()
+    date[:2], seg[:2] = dg.DATE_LO, 0
+    fk = np.where(rng.random(npr) < 0.7, rng.choice(key, npr), rng.integers(-2**31, 2**31, npr))
+    fk[:4] = [-2**31, 2**31 - 1, key.min(), key.max()]
+    j = dg.JoinInput(key.astype(np.int32), date, seg, fk.astype(np.int32), j.p_price, j.p_disc, j.date_lt, j.seg_eq)
+    params = params_for(nq, 33)
+    params[0] = (dg.DATE_HI + 1, 0)
+    b, p = device(torch_cuda, j)
+    got = engine.join_multi(b, p, len(key), npr, params)
+    for g, w in zip(got, oracle_answers(j, params)):
+        assert tuple(g[f] for f in FIELDS) == w
+        assert g["reruns"] == 0
+
+
+@pytest.mark.parametrize("step", [1, 5000])
+def test_join_multi_many_rows_per_warp(engine, torch_cuda, step):
+    """More matching rows per warp than its shared-memory accumulators may take between two flushes, all of one class
+    and with the largest summands."""
+    nb, npr = 400_000, 24_000_000
+    j = dg.gen_join(nb, npr, seed=41)
+    j.b_seg[:] = 3
+    j.b_date[:] = dg.DATE_LO
+    j.p_price[:] = 2**31 - 1
+    j.p_disc[:] = 1
+    j = dg.JoinInput(j.b_key * step, j.b_date, j.b_seg, j.p_fk * step, j.p_price, j.p_disc, j.date_lt, j.seg_eq)
+    params = [(dg.DATE_HI, 3), (dg.DATE_LO, 3), (dg.DATE_HI, 2)]
+    b, p = device(torch_cuda, j)
+    got = engine.join_multi(b, p, nb, npr, params)
+    for g, w in zip(got, oracle_answers(j, params)):
+        assert tuple(g[f] for f in FIELDS) == w
