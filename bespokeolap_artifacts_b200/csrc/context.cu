@@ -78,6 +78,17 @@ int consume_device_errors(bo_ctx* ctx, uint32_t* bits_out) {
   return BO_OK;
 }
 
+int read_result(bo_ctx* ctx, const char* op, void* host, const void* dev, size_t bytes) {
+  void* stage = nullptr;
+  int rc = host_stage(ctx, bytes, &stage);
+  if (rc) return rc;
+  BO_CUDA(ctx, cudaMemcpyAsync(stage, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  uint32_t bits = 0;
+  if ((rc = consume_device_errors(ctx, &bits))) return rc;  // synchronises the stream
+  std::memcpy(host, stage, bytes);
+  return device_error_status(ctx, bits, op);
+}
+
 int device_error_status(bo_ctx* ctx, uint32_t bits, const char* op) {
   if (bits == 0) return BO_OK;
   if (bits & kErrSpinTimeout)

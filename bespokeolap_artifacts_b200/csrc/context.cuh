@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <string>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "bespoke_gpu.h"
@@ -82,6 +83,10 @@ void destroy_host_work(bo_ctx* ctx);
 int after_launch(bo_ctx* ctx, const char* what);
 // Reads and clears the device error word (call only after a stream sync).
 int consume_device_errors(bo_ctx* ctx, uint32_t* bits_out);
+// A call's result record and the error word in one synchronisation: both are
+// copied to pinned memory, so neither copy waits for the other (a copy to
+// pageable memory synchronises by itself: 15 us more per call).
+int read_result(bo_ctx* ctx, const char* op, void* host, const void* dev, size_t bytes);
 // Maps error bits to a status code with a message.
 int device_error_status(bo_ctx* ctx, uint32_t bits, const char* op);
 // Blocks per SM from the occupancy calculator, cached per kernel.
@@ -133,6 +138,25 @@ int radix_topk_pairs(bo_ctx* ctx, const unsigned long long* keys, const uint32_t
                      const unsigned long long* n_dev, int key_bits, int k, unsigned long long* cand_keys,
                      uint32_t* cand_vals, unsigned long long* tmp_keys, uint32_t* tmp_vals, int lo_bits,
                      const unsigned long long* hi_max_dev);
+
+// Launches a kernel that may start while the previous kernel on the stream
+// still runs (programmatic dependent launch); the kernel itself waits
+// (pdl_wait) before it reads that kernel's output.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*k)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
+                             Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+}
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 // Column pointers must be 32-byte aligned: the scans use 256-bit vector loads.

@@ -67,7 +67,7 @@ struct GbMeta {
   int32_t cap_log2;
   uint32_t overflow;
   uint32_t done;
-  uint32_t pad;
+  uint32_t no_filter;                 // dense form: the Bloom filter was not filled
   unsigned long long joined;          // joined (surviving) B rows
   unsigned long long distinct;        // groups inserted into the global table
   unsigned long long n_out;           // compacted groups (sort key count)
@@ -715,6 +715,671 @@ __global__ void __launch_bounds__(kPartBlock) gb_part_agg_kernel(const uint4* __
   if (lane == 0 && cmaxc) atomicMax(&meta->inv_max, cmaxc);
 }
 
+// ============================================================ dense form ==
+// Aggregation by a_id itself instead of a hash table: one entry per id in [0,
+// a_id_max], where those fit the memory of the group table (gb_dense_fits).  A
+// survivor then costs L2 atomics without a returned value (the hash table: a
+// CAS round trip, then an add and a min), A's mask is applied to ids instead of
+// rows, and the top k comes out of one pass over the entries.
+//   cfilter  C rows -> one code byte per row (0: fails; else 1 + year -
+//            year_lo), and the 128 KB Bloom filter of the passing ids;
+//   scan     few C rows pass (gd_scan_kernel, one block per SM): the filter sits
+//            in shared memory (a random word costs about 3.4 bank cycles a warp
+//            there, 32 tag lookups a warp through L1), its hits queue per warp,
+//            and only rows whose code byte confirms them load their a_id.  Many
+//            pass (gd_scan_all_kernel): no filter, every row reads its code byte
+//            and streams its a_id.  The device decides, the other one returns;
+//   collect  entries of A's ids: groups, joined rows, the k best of each block,
+//            and in the last block the k best of all and the result record;
+//   years    (counts alone) B once more for the smallest years of the k groups.
+// Entries are {count, smallest year} pairs while those stay well inside L2, and
+// counts alone beyond (kGdPairIds): half the memory, half the atomics.
+// Measured (B200, device time): A 2.5M, B 36M, C 4M, 1% of C: 92 us (cfilter 12,
+// scan 54, collect 21) against 137 us of the hash form; A 25M, B 60M, C 4M, half
+// of C: 810 against 3300 us partitioned by hash (scan 1810, scatter 800, ...).
+constexpr int kGdBlock = 1024;
+constexpr int kGdWarps = kGdBlock / 32;
+constexpr int kGdLog2Words = 15;  // Bloom filter: 2^15 words = 128 KB
+constexpr uint32_t kGdWords = 1u << kGdLog2Words;
+constexpr uint32_t kGdFilterBytes = kGdWords * 4;
+constexpr int kGdFlushAt = 64;
+constexpr int kGdQueue = 320;     // per-warp candidate queue: up to kGdFlushAt left over + one step of 256 rows
+constexpr int kGdResolveR = 2;
+constexpr int kGdLocalSlots = 512;
+constexpr size_t kGdSmem = kGdFilterBytes + (size_t)kGdWarps * kGdQueue * 8;
+// The filter is used while at most a quarter of its bits can be set.
+constexpr unsigned long long kGdFilterKeys = (unsigned long long)kGdWords * 32 / 8;
+// B rows below which copying the filter to every SM costs more than it saves.
+constexpr int64_t kGdFilterRows = 1 << 20;
+// Smallest years are kept as the largest (kGdYearTop - code), 0 where there is
+// none, so that entries start as zero bytes.
+constexpr uint32_t kGdYearTop = 255;
+// Counts are added to in passes over ids that each have at most this many bytes
+// of them, half of L2 (25M ids, 100 MB: one pass 705 us, two 633, three 705;
+// 12.5M ids, 50 MB: two passes cost 8% of the query).
+constexpr int64_t kGdPassBytes = 64 << 20;
+constexpr int64_t kGdPairIds = 8 << 20;  // 64 MB of pairs: half of L2
+
+__device__ __forceinline__ void gd_bloom_pos(uint32_t key, uint32_t& word, uint32_t& bits) {
+  const uint32_t h = key * 0x9E3779B1u;
+  word = h >> (32 - kGdLog2Words);
+  bits = (1u << (h & 31u)) | (1u << ((h >> 5) & 31u));
+}
+
+// Thread w owns C rows [32w, 32w + 32): 32 code bytes.
+__global__ void __launch_bounds__(256) gd_cfilter_kernel(bo_gb_c_cols c, CatSet cats, int32_t year_lo, int32_t year_hi,
+                                                         uint8_t* __restrict__ code, uint32_t* __restrict__ cbits,
+                                                         uint32_t* __restrict__ bloom, uint4* __restrict__ entries,
+                                                         int64_t entry_vecs, GbMeta* meta, const float* pred,
+                                                         int32_t host_log2, int32_t max_log2) {
+  __shared__ uint32_t catmask[2048];
+  pdl_launch_dependents();
+  for (int i = threadIdx.x; i < 2048; i += blockDim.x) catmask[i] = 0;
+  __syncthreads();
+  if (threadIdx.x < cats.n) atomicOr(&catmask[cats.v[threadIdx.x] >> 5], 1u << (cats.v[threadIdx.x] & 31u));
+  __syncthreads();
+  const int64_t n = c.n_rows;
+  const int64_t words = (n + 31) / 32;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (tid == 0) meta->cap_log2 = gb_presize_log2(pred, host_log2, max_log2);
+  // A table that would fill the filter many times over is not put into it: 256
+  // rows spread over the table, the same for every block, tell (4M rows of
+  // which half pass: 52 -> 24 us).
+  if (bloom && n > 4 * (int64_t)kGdFilterKeys) {
+    const int64_t r = (int64_t)(((uint64_t)hash32(threadIdx.x) * (uint64_t)n) >> 32);
+    const uint32_t cv = c.category[r];
+    const int32_t y = c.year[r];
+    const int got = __syncthreads_count(((catmask[cv >> 5] >> (cv & 31u)) & 1u) && y >= year_lo && y <= year_hi);
+    if ((int64_t)got * n > 256 * 4 * (int64_t)kGdFilterKeys) {
+      bloom = nullptr;
+      if (tid == 0) meta->no_filter = 1;
+    }
+  }
+  for (int64_t i = tid; i < entry_vecs; i += stride) entries[i] = make_uint4(0, 0, 0, 0);
+  uint32_t passed = 0;
+  for (int64_t w = tid; w < words; w += stride) {
+    const int64_t r0 = w * 32;
+    uint32_t bits = 0;
+    if (r0 + 32 <= n) {
+      int8v cat[2];
+      cat[0] = ld_stream_v8(c.category + r0);
+      cat[1] = ld_stream_v8(c.category + r0 + 16);
+      uint32_t cw[8];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int8v y = ld_stream_v8(c.year + r0 + 8 * q);
+        cw[2 * q] = cw[2 * q + 1] = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int row = 8 * q + k;
+          const uint32_t word = (uint32_t)cat[row >> 4].v[(row & 15) >> 1];
+          const uint32_t cv = (row & 1) ? (word >> 16) : (word & 0xffffu);
+          const bool ok = ((catmask[cv >> 5] >> (cv & 31u)) & 1u) && y.v[k] >= year_lo && y.v[k] <= year_hi;
+          bits |= (uint32_t)ok << row;
+          cw[row >> 2] |= ok ? (uint32_t)(y.v[k] - year_lo + 1) << (8 * (row & 3)) : 0u;
+        }
+      }
+      uint4* dst = reinterpret_cast<uint4*>(code + r0);
+      dst[0] = make_uint4(cw[0], cw[1], cw[2], cw[3]);
+      dst[1] = make_uint4(cw[4], cw[5], cw[6], cw[7]);
+    } else {
+      for (int k = 0; k < 32 && r0 + k < n; ++k) {
+        const uint32_t cv = c.category[r0 + k];
+        const int32_t y = c.year[r0 + k];
+        const bool ok = ((catmask[cv >> 5] >> (cv & 31u)) & 1u) && y >= year_lo && y <= year_hi;
+        bits |= (uint32_t)ok << k;
+        code[r0 + k] = ok ? (uint8_t)(y - year_lo + 1) : 0;
+      }
+    }
+    cbits[w] = bits;
+    passed += __popc(bits);
+    if (!bloom) continue;
+    while (bits) {
+      const int k = __ffs(bits) - 1;
+      bits &= bits - 1;
+      uint32_t bw, bb;
+      gd_bloom_pos((uint32_t)(r0 + k), bw, bb);
+      if ((__ldcg(bloom + bw) & bb) != bb) atomicOr(bloom + bw, bb);  // a filling filter costs reads, not atomics
+    }
+  }
+  __shared__ uint32_t part[8];
+  passed = warp_sum_u32(passed);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = passed;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += part[i];
+    if (t) atomicAdd(&meta->c_pass, (unsigned long long)t);
+  }
+}
+
+// Whether the filtered scan runs.
+__device__ __forceinline__ bool gd_filtered(const GbMeta* meta, bool has_filter) {
+  return has_filter && !__ldcg(&meta->no_filter) && __ldcg(&meta->c_pass) <= kGdFilterKeys;
+}
+
+// A block's pre-aggregation of heavy hitters, as gb_scan_kernel's, which a warp
+// leaves once it has seen that fewer than a quarter of its keys are there.
+struct GdLocal {
+  uint32_t key[kGdLocalSlots], cnt[kGdLocalSlots], year[kGdLocalSlots];
+  __device__ __forceinline__ void clear() {
+    for (int i = threadIdx.x; i < kGdLocalSlots; i += blockDim.x) {
+      key[i] = 0xffffffffu;
+      cnt[i] = 0;
+      year[i] = 0;
+    }
+  }
+};
+
+struct GdTries {
+  uint32_t tries = 0, hits = 0;
+};
+
+// True if the local table took the key.
+template <bool kYear>
+__device__ __forceinline__ bool gd_add_local(GdLocal& l, GdTries& t, uint32_t a, uint32_t year) {
+  const uint32_t h = hash32(a);
+  ++t.tries;
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const int sl = (int)((h + p) & (kGdLocalSlots - 1));
+    const uint32_t old = atomicCAS(&l.key[sl], 0xffffffffu, a);
+    if (old == 0xffffffffu || old == a) {
+      t.hits += old == a;
+      atomicAdd(&l.cnt[sl], 1u);
+      if (kYear) atomicMax(&l.year[sl], year);
+      return true;
+    }
+  }
+  return false;
+}
+
+// Whether the warp keeps to the local table (asked by all lanes together).
+__device__ __forceinline__ bool gd_keep_local(const GdTries& t) {
+  const uint32_t tries = __reduce_add_sync(0xffffffffu, t.tries), hits = __reduce_add_sync(0xffffffffu, t.hits);
+  return tries < 512u || hits * 4u >= tries;
+}
+
+// Eight consecutive ids of this lane in a warp's step of 256 rows; -1 past the
+// end (no partner).
+__device__ __forceinline__ void gd_load8(const int32_t* col, int64_t n, int64_t st, int32_t (&out)[8]) {
+  const int64_t r0 = st * 256 + (threadIdx.x & 31) * 8;
+  if (r0 + 8 <= n) {
+    const int8v v = ld_first_v8(col + r0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = v.v[k];
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) out[k] = r0 + k < n ? col[r0 + k] : -1;
+  }
+}
+
+// One survivor into its entry: a pair's count and year, or a count alone.
+template <bool kYear>
+__device__ __forceinline__ void gd_add(uint32_t* entries, uint32_t a, uint32_t cnt, uint32_t year) {
+  if (kYear) {
+    atomicAdd(entries + 2 * (size_t)a, cnt);
+    atomicMax(entries + 2 * (size_t)a + 1, year);
+  } else {
+    atomicAdd(entries + a, cnt);
+  }
+}
+
+template <bool kYear>
+__device__ __forceinline__ void gd_flush_local(const GdLocal& l, uint32_t* entries) {
+  __syncthreads();
+  for (int i = threadIdx.x; i < kGdLocalSlots; i += blockDim.x)
+    if (l.key[i] != 0xffffffffu) gd_add<kYear>(entries, l.key[i], l.cnt[i], l.year[i]);
+}
+
+template <bool kYear>
+__global__ void __launch_bounds__(kGdBlock, 1) gd_scan_kernel(bo_gb_b_cols b, int64_t n_c, int32_t a_id_max,
+                                                              const uint8_t* __restrict__ code,
+                                                              const uint32_t* __restrict__ bloom,
+                                                              const GbMeta* __restrict__ meta,
+                                                              uint32_t* __restrict__ entries, uint32_t* err) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (!gd_filtered(meta, true)) return;
+  extern __shared__ __align__(128) uint32_t gd_smem[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ GdLocal local;
+  local.clear();
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    mbar_arrive_expect_tx(&bar, kGdFilterBytes);
+    bulk_copy_g2s(gd_smem, bloom, kGdFilterBytes / 2, &bar);
+    bulk_copy_g2s(gd_smem + kGdWords / 2, bloom + kGdWords / 2, kGdFilterBytes / 2, &bar);
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = b.n_rows;
+  const int64_t steps = (n + 255) / 256;
+  const int64_t nwarps = (int64_t)gridDim.x * kGdWarps;
+  const uint32_t nc = (uint32_t)n_c;  // n_c < 2^31; ids outside [0, n_c) have no partner
+  int64_t st = (int64_t)blockIdx.x * kGdWarps + warp;
+  int32_t n1[8], n2[8];  // the next two steps' ids, in flight
+  if (st < steps) gd_load8(b.c_id, n, st, n1);
+  if (st + nwarps < steps) gd_load8(b.c_id, n, st + nwarps, n2);
+  __syncthreads();
+  // Without the filter (a timed-out copy, never expected) every word is taken as all ones: same answer.
+  const uint32_t pass = mbar_wait_bounded(&bar, 0, kWaitLimitNs) ? 0u : 0xffffffffu;
+  if (pass) raise_error(err, kErrSpinTimeout);
+  uint32_t* qc = gd_smem + kGdWords + warp * kGdQueue * 2;
+  uint32_t* qr = qc + kGdQueue;
+  uint32_t qn = 0;  // queued candidates (warp-uniform)
+  GdTries tries;
+  bool use_local = true;
+  auto resolve = [&]() {
+    __syncwarp();
+    for (uint32_t i0 = 0; i0 < qn; i0 += 32 * kGdResolveR) {
+      uint32_t c[kGdResolveR], row[kGdResolveR], y[kGdResolveR];
+      int32_t a[kGdResolveR];
+#pragma unroll
+      for (int r = 0; r < kGdResolveR; ++r) {
+        const uint32_t i = i0 + r * 32 + lane;
+        c[r] = i < qn ? qc[i] : 0xffffffffu;
+        row[r] = i < qn ? qr[i] : 0u;
+        y[r] = c[r] < nc ? __ldg(code + c[r]) : 0u;
+      }
+#pragma unroll
+      for (int r = 0; r < kGdResolveR; ++r) a[r] = y[r] ? __ldg(b.a_id + row[r]) : -1;
+#pragma unroll
+      for (int r = 0; r < kGdResolveR; ++r) {
+        if (a[r] < 0 || a[r] > a_id_max) continue;
+        const uint32_t yr = kGdYearTop - y[r];
+        if (use_local && gd_add_local<kYear>(local, tries, (uint32_t)a[r], yr)) continue;
+        gd_add<kYear>(entries, (uint32_t)a[r], 1u, yr);
+      }
+    }
+    qn = 0;
+    if (use_local) use_local = gd_keep_local(tries);
+    __syncwarp();
+  };
+  // One step's ids: tests, then its few hits into the queue, one per lane and
+  // round (a lane rarely has two), and the ids of two steps on requested into
+  // the same registers.
+  auto step = [&](int32_t (&cid)[8]) {
+    uint32_t hit = 0;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+      const uint32_t h = (uint32_t)cid[k] * 0x9E3779B1u;
+      const uint32_t x = gd_smem[h >> (32 - kGdLog2Words)] | pass;
+      hit = (hit << 1) | (__funnelshift_r(x, x, h) & __funnelshift_r(x, x, h >> 5) & 1u);
+    }
+    const uint32_t r0 = (uint32_t)(st * 256) + lane * 8;
+    for (uint32_t who = __ballot_sync(0xffffffffu, hit != 0); who; who = __ballot_sync(0xffffffffu, hit != 0)) {
+      if (hit) {
+        const int k = __ffs(hit) - 1;
+        hit &= hit - 1;
+        const int32_t c01 = k & 1 ? cid[1] : cid[0], c23 = k & 1 ? cid[3] : cid[2];
+        const int32_t c45 = k & 1 ? cid[5] : cid[4], c67 = k & 1 ? cid[7] : cid[6];
+        const int32_t c03 = k & 2 ? c23 : c01, c47 = k & 2 ? c67 : c45;
+        const uint32_t pos = qn + __popc(who & ((1u << lane) - 1u));
+        qc[pos] = (uint32_t)(k & 4 ? c47 : c03);
+        qr[pos] = r0 + k;
+      }
+      qn += __popc(who);
+    }
+    if (st + 2 * nwarps < steps) gd_load8(b.c_id, n, st + 2 * nwarps, cid);
+    if (qn >= kGdFlushAt) resolve();
+    st += nwarps;
+  };
+  while (st < steps) {
+    step(n1);
+    if (st < steps) step(n2);
+  }
+  if (qn) resolve();
+  gd_flush_local<kYear>(local, entries);
+  if (pass) mbar_wait_bounded(&bar, 0, kWaitLimitNs);  // the copy may still be in flight
+}
+
+// Every row: its code byte (random, from L2), its a_id (streamed), its atomics.
+// Counts alone need no year, so a bit of the exact bitmap does, an eighth of
+// the bytes, of which L1 keeps a good part.  Bound by one L1-to-L2 request per
+// cycle and SM (50% busy): 633 us for 60M rows of which half join (740 us with
+// code bytes, in one pass over all ids).
+constexpr int kGaBlock = 256;
+
+template <bool kYear>
+__global__ void __launch_bounds__(kGaBlock, 8)
+    gd_scan_all_kernel(bo_gb_b_cols b, int64_t n_c, int32_t id_lo, int32_t id_hi, const uint8_t* __restrict__ code,
+                       const uint32_t* __restrict__ cbits, const GbMeta* __restrict__ meta, bool has_filter,
+                       uint32_t* __restrict__ entries) {
+  pdl_launch_dependents();
+  pdl_wait();
+  if (gd_filtered(meta, has_filter)) return;
+  __shared__ GdLocal local;
+  local.clear();
+  __syncthreads();
+  const int64_t n = b.n_rows;
+  const int64_t steps = (n + 255) / 256;
+  const int64_t nwarps = (int64_t)gridDim.x * (kGaBlock / 32);
+  const uint32_t nc = (uint32_t)n_c;
+  GdTries tries;
+  bool use_local = true;
+  for (int64_t st = (int64_t)blockIdx.x * (kGaBlock / 32) + (threadIdx.x >> 5); st < steps; st += nwarps) {
+    int32_t cid[8], aid[8];
+    gd_load8(b.c_id, n, st, cid);
+    gd_load8(b.a_id, n, st, aid);
+    uint32_t y[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const bool in = (uint32_t)cid[k] < nc && aid[k] >= id_lo && aid[k] <= id_hi;
+      if (kYear) y[k] = in ? __ldg(code + cid[k]) : 0u;
+      else y[k] = in ? (__ldg(cbits + (cid[k] >> 5)) >> (cid[k] & 31)) & 1u : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (!y[k]) continue;
+      if (use_local && gd_add_local<kYear>(local, tries, (uint32_t)aid[k], kGdYearTop - y[k])) continue;
+      gd_add<kYear>(entries, (uint32_t)aid[k], 1u, kGdYearTop - y[k]);
+    }
+    if (use_local) use_local = gd_keep_local(tries);
+  }
+  gd_flush_local<kYear>(local, entries);
+}
+
+constexpr int kGcBlock = 256;
+constexpr int kGcPer = 8;                  // consecutive ids per thread and step
+constexpr int kGcTile = kGcBlock * kGcPer;
+constexpr int kGcKeep = kGcTile;           // candidates kept between steps before they are cut to k
+constexpr int kGcBuf = kGcKeep + kGcTile;
+
+// Upper bound of the k-th smallest of the block's keys, k <= 64: the k-th
+// smallest of the minima of 64 groups of four threads (k keys do not exceed
+// it; ~0 if fewer groups have a key).  All threads of the block call it.
+__device__ __forceinline__ unsigned long long gc_bound(unsigned long long mine, int k) {
+  __shared__ unsigned long long gmin[64], bound;
+  for (int o = 1; o < 4; o <<= 1) {
+    const unsigned long long x = __shfl_xor_sync(0xffffffffu, mine, o);
+    mine = x < mine ? x : mine;
+  }
+  if ((threadIdx.x & 3) == 0) gmin[threadIdx.x >> 2] = mine;
+  if (threadIdx.x == 0) bound = ~0ull;
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    const unsigned long long v = gmin[threadIdx.x];
+    int r = 0;
+#pragma unroll 16
+    for (int i = 0; i < 64; ++i) r += gmin[i] < v;
+    if (r == k - 1) bound = v;  // unique unless ~0
+  }
+  __syncthreads();
+  return bound;
+}
+
+// The k smallest of the m <= kGcBuf unique keys in buf, ascending, to its front.
+// All threads of the block call it.  Few keys: each thread ranks one; more: cut
+// down by the bound of gc_bound first (m keys leave at most k * ceil(m / 64)).
+__device__ __forceinline__ uint32_t gc_cut(unsigned long long* buf, uint32_t m, int k) {
+  __shared__ uint32_t left;
+  while (m > (uint32_t)kGcBlock) {
+    unsigned long long own[kGcBuf / kGcBlock], mine = ~0ull;
+#pragma unroll
+    for (int i = 0; i < kGcBuf / kGcBlock; ++i) {
+      const uint32_t at = i * kGcBlock + threadIdx.x;
+      own[i] = at < m ? buf[at] : ~0ull;
+      mine = own[i] < mine ? own[i] : mine;
+    }
+    if (threadIdx.x == 0) left = 0;
+    const unsigned long long bound = gc_bound(mine, k);  // also: all keys are in registers
+#pragma unroll
+    for (int i = 0; i < kGcBuf / kGcBlock; ++i)
+      if (own[i] <= bound && own[i] != ~0ull) buf[atomicAdd(&left, 1u)] = own[i];
+    __syncthreads();
+    if (left == m) break;  // cannot shrink further (k near 64 of few hundred keys): ranked below
+    m = left;
+    __syncthreads();
+  }
+  unsigned long long v[kGcBuf / kGcBlock];
+  uint32_t r[kGcBuf / kGcBlock];
+  const int per = (int)((m + kGcBlock - 1) / kGcBlock);
+  for (int i = 0; i < per; ++i) {
+    const uint32_t at = i * kGcBlock + threadIdx.x;
+    v[i] = at < m ? buf[at] : ~0ull;
+    r[i] = 0;
+    for (uint32_t j = 0; j < m; ++j) r[i] += buf[j] < v[i];
+  }
+  __syncthreads();
+  for (int i = 0; i < per; ++i)
+    if (v[i] != ~0ull && r[i] < (uint32_t)k) buf[r[i]] = v[i];
+  __syncthreads();
+  return m < (uint32_t)k ? m : (uint32_t)k;
+}
+
+// kParts: also counts groups per hash partition (the partitioned form's rule
+// for too few partitions).  kPairs: entries are {count, year}.
+template <bool kParts, bool kPairs>
+__global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t* __restrict__ entries, int64_t n_ids,
+                                                              const uint32_t* __restrict__ amask, GbMeta* meta,
+                                                              int32_t year_lo, int k, int wa, unsigned long long cmax,
+                                                              uint32_t* __restrict__ part_counts, uint32_t n_parts,
+                                                              uint32_t shift, unsigned long long* __restrict__ cand,
+                                                              bo_gb_result* __restrict__ out) {
+  extern __shared__ uint32_t hist[];  // kParts: n_parts counters
+  __shared__ unsigned long long buf[kGcBuf];
+  __shared__ uint32_t count_s, over_s;
+  __shared__ unsigned long long red[2][kGcBlock / 32];
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) count_s = over_s = 0;
+  if (kParts)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kGcBlock) hist[i] = 0;
+  pdl_wait();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long limit = k > 0 ? ~0ull : 0ull;  // only keys below it can be among the k best
+  uint32_t groups = 0;
+  unsigned long long joined = 0;
+  // This thread's eight counts of tile t, zero where the id is not one of A's.
+  auto load = [&](int64_t t, uint32_t (&c)[kGcPer]) {
+    const int64_t id0 = t * kGcTile + threadIdx.x * kGcPer;
+    if (id0 + kGcPer <= n_ids) {
+      if (kPairs) {
+        const int8v v0 = ld_first_v8(entries + 2 * id0), v1 = ld_first_v8(entries + 2 * id0 + 8);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          c[j] = (uint32_t)v0.v[2 * j];
+          c[4 + j] = (uint32_t)v1.v[2 * j];
+        }
+      } else {
+        const int8v v = ld_first_v8(entries + id0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) c[j] = (uint32_t)v.v[j];
+      }
+      const uint32_t am = __ldg(amask + (id0 >> 5)) >> (id0 & 31);  // id0 is a multiple of eight
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j)
+        if (!((am >> j) & 1u)) c[j] = 0;
+    } else {
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j) {
+        const int64_t id = id0 + j;
+        c[j] = 0;
+        if (id < n_ids && ((__ldg(amask + (id >> 5)) >> (id & 31)) & 1u)) c[j] = entries[kPairs ? 2 * id : id];
+      }
+    }
+  };
+  // Appends this thread's keys below the limit to the candidates; the first
+  // call of a phase takes the limit from the keys themselves.  (some: false
+  // where the caller knows that no key of this thread is below it.)
+  auto keep = [&](const unsigned long long (&key)[kGcPer], bool first, bool some) {
+    if (first && k > 0) {
+      unsigned long long mine = ~0ull;
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j) mine = key[j] < mine ? key[j] : mine;
+      const unsigned long long b = gc_bound(mine, k);
+      if (b != ~0ull) limit = b + 1;
+    }
+    uint32_t take = 0;
+    if (some) {
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j) take |= (uint32_t)(key[j] < limit) << j;
+    }
+    if (!__syncthreads_or(take != 0)) return;  // uniform
+    if (__any_sync(0xffffffffu, take != 0)) {
+      uint32_t total, pos = 0;
+      const uint32_t before = warp_exclusive_scan(__popc(take), total);
+      if (lane == 0) pos = atomicAdd(&count_s, total);
+      pos = __shfl_sync(0xffffffffu, pos, 0) + before;
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j)
+        if ((take >> j) & 1u) buf[pos++] = key[j];
+    }
+    __syncthreads();
+    const uint32_t m = count_s;
+    if (m > (uint32_t)kGcKeep) {  // uniform
+      const uint32_t left = gc_cut(buf, m, k);
+      if (threadIdx.x == 0) count_s = left;
+      limit = buf[k - 1];
+    }
+    __syncthreads();
+  };
+  const int64_t tiles = (n_ids + kGcTile - 1) / kGcTile;
+  // Contiguous runs of tiles: a block meets ids in ascending order.
+  const int64_t per = (tiles + gridDim.x - 1) / gridDim.x;
+  const int64_t t0 = blockIdx.x * per, t1 = t0 + per < tiles ? t0 + per : tiles;
+  uint32_t n1[kGcPer], n2[kGcPer];  // the next two tiles, in flight
+  if (t0 < t1) load(t0, n1);
+  if (t0 + 1 < t1) load(t0 + 1, n2);
+  __syncthreads();
+  auto step = [&](int64_t t, uint32_t (&c)[kGcPer]) {
+    const uint32_t id0 = (uint32_t)(t * kGcTile) + threadIdx.x * kGcPer;
+    // Counts below the limit's cannot be among the best: most threads stop here.
+    const unsigned long long need = limit == ~0ull ? 1ull : cmax - (limit >> wa);
+    uint32_t most = 0;
+#pragma unroll
+    for (int j = 0; j < kGcPer; ++j) {
+      groups += c[j] != 0;
+      joined += c[j];
+      most = c[j] > most ? c[j] : most;
+      if (kParts && c[j]) atomicAdd(hist + (shift >= 32 ? 0u : hash32(id0 + j) >> shift), 1u);
+    }
+    const bool some = most >= need && most > 0;
+    unsigned long long key[kGcPer];
+#pragma unroll
+    for (int j = 0; j < kGcPer; ++j) key[j] = some && c[j] ? ((cmax - c[j]) << wa) | (id0 + j) : ~0ull;
+    if (t + 2 < t1) load(t + 2, c);
+    keep(key, t == t0, some);
+  };
+  for (int64_t t = t0; t < t1; t += 2) {
+    step(t, n1);
+    if (t + 1 < t1) step(t + 1, n2);
+  }
+  uint32_t mine = k > 0 ? gc_cut(buf, count_s, k) : 0;
+  if (threadIdx.x < (uint32_t)k)
+    cand[(size_t)blockIdx.x * k + threadIdx.x] = threadIdx.x < mine ? buf[threadIdx.x] : ~0ull;
+  if (kParts)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kGcBlock)
+      if (hist[i]) atomicAdd(part_counts + i, hist[i]);
+  groups = warp_sum_u32(groups);
+  joined = (unsigned long long)warp_sum_i64((int64_t)joined);
+  if (lane == 0) {
+    red[0][warp] = groups;
+    red[1][warp] = joined;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long g = 0, jr = 0;
+    for (int w = 0; w < kGcBlock / 32; ++w) {
+      g += red[0][w];
+      jr += red[1][w];
+    }
+    if (g) atomicAdd(&meta->n_out, g);
+    if (jr) atomicAdd(&meta->joined, jr);
+  }
+  if (!last_block(&meta->done)) return;
+  if (kParts)
+    for (uint32_t i = threadIdx.x; i < n_parts; i += kGcBlock)
+      if (__ldcg(part_counts + i) > kPartMaxGroups) over_s = 1;
+  if (gridDim.x > 1 && k > 0) {
+    if (threadIdx.x == 0) count_s = 0;
+    limit = ~0ull;
+    __syncthreads();
+    const uint32_t all = gridDim.x * (uint32_t)k;
+    for (uint32_t i0 = 0; i0 < all; i0 += kGcTile) {
+      unsigned long long key[kGcPer];
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j) {
+        const uint32_t i = i0 + j * kGcBlock + threadIdx.x;
+        key[j] = i < all ? __ldcg(cand + i) : ~0ull;
+      }
+      keep(key, i0 == 0, true);
+    }
+    mine = gc_cut(buf, count_s, k);
+  }
+  __syncthreads();
+  const unsigned long long n = __ldcg(&meta->n_out);
+  if (threadIdx.x < mine) {
+    const unsigned long long key = buf[threadIdx.x];
+    const uint32_t id = (uint32_t)(key & ((1ull << wa) - 1ull));
+    bo_gb_row r;
+    r.a_id = (int32_t)id;
+    r.min_year = kPairs ? year_lo + (int32_t)(kGdYearTop - entries[2 * (size_t)id + 1]) - 1 : 0x7fffffff;
+    r.count = (int64_t)(cmax - (key >> wa));
+    out->rows[threadIdx.x] = r;
+  }
+  if (threadIdx.x == 0) {
+    const int32_t cl = __ldcg(&meta->cap_log2);
+    const unsigned long long cap = 1ull << cl;
+    out->n_groups = (int64_t)n;
+    out->joined_rows = (int64_t)__ldcg(&meta->joined);
+    out->c_qualifying = (int64_t)__ldcg(&meta->c_pass);
+    out->capacity_log2 = cl;
+    // The table a prediction sized (or a partition's) would have been too full.
+    out->overflowed = kParts ? (int32_t)over_s : (int32_t)(n > cap - (cap >> 3));
+    out->reruns = 0;
+    out->mode = kParts ? 2 : 1;
+    out->n_rows_out = (int32_t)mine;
+    out->exact_distinct = 0;
+  }
+}
+
+// Counts alone: the smallest years of the result's groups.  Bound by streaming
+// B's a_ids; a row of one of the at most 64 groups is rare.
+__global__ void __launch_bounds__(256) gd_years_kernel(bo_gb_b_cols b, int64_t n_c, int32_t year_lo,
+                                                       const uint8_t* __restrict__ code,
+                                                       bo_gb_result* __restrict__ out) {
+  pdl_wait();
+  constexpr int kBits = 1 << 16;  // one hashed bit per group: at most one other row in a thousand gets past it
+  __shared__ uint32_t bits[kBits / 32];
+  __shared__ int32_t key[BO_GB_MAX_K];
+  const int rows = out->n_rows_out;
+  for (int i = threadIdx.x; i < kBits / 32; i += 256) bits[i] = 0;
+  __syncthreads();
+  if (threadIdx.x < rows) {
+    const int32_t a = out->rows[threadIdx.x].a_id;
+    key[threadIdx.x] = a;
+    const uint32_t h = ((uint32_t)a * 0x9E3779B1u) >> 16;
+    atomicOr(bits + (h >> 5), 1u << (h & 31u));
+  }
+  __syncthreads();
+  const int64_t n = b.n_rows;
+  const int64_t steps = (n + 255) / 256;
+  for (int64_t st = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); st < steps; st += (int64_t)gridDim.x * 8) {
+    int32_t a[8];
+    gd_load8(b.a_id, n, st, a);
+    uint32_t hit = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t h = ((uint32_t)a[j] * 0x9E3779B1u) >> 16;
+      hit |= ((bits[h >> 5] >> (h & 31u)) & 1u) << j;
+    }
+    if (!hit) continue;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (!((hit >> j) & 1u)) continue;
+      const int64_t r = st * 256 + (threadIdx.x & 31) * 8 + j;
+      if (r >= n) continue;
+      for (int i = 0; i < rows; ++i) {
+        if (key[i] != a[j]) continue;
+        const int32_t c = b.c_id[r];
+        const uint32_t y = (uint32_t)c < (uint32_t)n_c ? __ldg(code + c) : 0u;
+        if (y) atomicMin(&out->rows[i].min_year, year_lo + (int32_t)y - 1);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ topk --
 __global__ void gb_topk_kernel(const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals,
                                GbMeta* meta, int k, int wa, unsigned long long cmax, int mode,
@@ -904,12 +1569,112 @@ int gb_aggregate_order(bo_ctx* ctx, const bo_gb_b_cols& b, const bo_gb_c_cols& c
   return after_launch(ctx, "gb_topk_kernel");
 }
 
+// The dense form takes a call whose entries (8 B per id) fit the group table's
+// slots and whose years fit a byte.  The presized form also wants at most one
+// id per two B rows: the entries are cleared and read once whatever joins,
+// which beyond that costs more than the small hash table of a selective query.
+bool gb_dense_fits(const bo_gb_b_cols& b, const bo_gb_params& prm, const GbWs& ws, bool partitioned) {
+  const int64_t ids = (int64_t)prm.a_id_max + 1;
+  if ((int64_t)prm.year_hi - prm.year_lo > 253 || ids > ((int64_t)1 << ws.max_log2)) return false;
+  return partitioned || ids <= std::max<int64_t>(b.n_rows / 2, 1 << 16);
+}
+
+// The dense form, asynchronous; n_parts == 0: presized from pred, else the
+// partitioned form with n_parts partitions.  *took is false when its
+// scratch cannot be had (the hash form then runs).
+int gb_dense(bo_ctx* ctx, const bo_gb_a_cols& a, const bo_gb_b_cols& b, const bo_gb_c_cols& c, const bo_gb_params& prm,
+             const GbWs& ws, const float* pred, uint32_t n_parts, uint32_t shift, bo_gb_result* out, bool* took) {
+  const bool parts = n_parts > 0;
+  const int64_t ids = (int64_t)prm.a_id_max + 1;
+  auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
+  const int64_t tiles = (ids + kGcTile - 1) / kGcTile;
+  const int gk = (int)std::min<int64_t>(tiles, (int64_t)ctx->num_sms * 3);  // all resident; few candidates to merge
+  const size_t meta_bytes = al(sizeof(GbMeta)), cnt_bytes = al(4 * (size_t)n_parts);
+  const size_t cand_bytes = al(8 * (size_t)BO_GB_MAX_K * gk), code_bytes = al((size_t)c.n_rows + 32);
+  void* base = nullptr;
+  *took = false;
+  if (region(ctx, "gb_dense", meta_bytes + kGdFilterBytes + cnt_bytes + cand_bytes + code_bytes, &base) != BO_OK) {
+    cudaGetLastError();
+    return BO_OK;
+  }
+  *took = true;
+  char* p = static_cast<char*>(base);
+  GbMeta* meta = reinterpret_cast<GbMeta*>(p);
+  uint32_t* bloom = reinterpret_cast<uint32_t*>(p + meta_bytes);
+  uint32_t* part_counts = reinterpret_cast<uint32_t*>(p + meta_bytes + kGdFilterBytes);
+  auto* cand = reinterpret_cast<unsigned long long*>(p + meta_bytes + kGdFilterBytes + cnt_bytes);
+  uint8_t* code = reinterpret_cast<uint8_t*>(p + meta_bytes + kGdFilterBytes + cnt_bytes + cand_bytes);
+  BO_CUDA(ctx, cudaMemsetAsync(p, 0, meta_bytes + kGdFilterBytes + cnt_bytes, ctx->stream));
+  const uint32_t* amask = prm.a_mask ? prm.a_mask : ws.amask;
+  int rc;
+  if (!prm.a_mask) {
+    BO_CUDA(ctx, cudaMemsetAsync(ws.amask, 0, 4 * (size_t)ws.mask_words, ctx->stream));
+    if (a.n_rows > 0) {
+      const void* ka = reinterpret_cast<const void*>(&gb_amask_kernel);
+      gb_amask_kernel<<<grid_res(ctx, ka, 256, 0, a.n_rows), 256, 0, ctx->stream>>>(a, prm.a_id_max, ws.amask,
+                                                                                    ctx->d_err);
+      if ((rc = after_launch(ctx, "gb_amask_kernel"))) return rc;
+    }
+  }
+  CatSet cs{};
+  cs.n = prm.n_categories;
+  for (int i = 0; i < prm.n_categories; ++i) cs.v[i] = prm.categories[i];
+  const bool filter = b.n_rows >= kGdFilterRows, pairs = ids <= kGdPairIds;
+  uint32_t* entries = reinterpret_cast<uint32_t*>(ws.slots);
+  const int64_t vecs = (ids * (pairs ? 8 : 4) + 15) / 16;
+  const void* kc = reinterpret_cast<const void*>(&gd_cfilter_kernel);
+  gd_cfilter_kernel<<<grid_res(ctx, kc, 256, 0, std::max<int64_t>((c.n_rows + 31) / 32, vecs / 8)), 256, 0,
+                      ctx->stream>>>(c, cs, prm.year_lo, prm.year_hi, code, ws.cbits, filter ? bloom : nullptr,
+                                     reinterpret_cast<uint4*>(entries), vecs, meta, pred, kGbMinCapLog2, ws.max_log2);
+  if ((rc = after_launch(ctx, "gd_cfilter_kernel"))) return rc;
+  const int64_t steps = (b.n_rows + 255) / 256;
+  const int64_t lanes = steps * 32;
+  if (filter) {
+    const auto ks = pairs ? &gd_scan_kernel<true> : &gd_scan_kernel<false>;
+    static bool ready[2] = {false, false};
+    if (!ready[pairs])
+      BO_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(ks), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kGdSmem));
+    ready[pairs] = true;
+    const int gs = (int)std::min<int64_t>(ctx->num_sms, (steps + kGdWarps - 1) / kGdWarps);
+    BO_CUDA(ctx, launch_dependent(ks, gs, kGdBlock, kGdSmem, ctx->stream, b, c.n_rows, prm.a_id_max,
+                                  (const uint8_t*)code, (const uint32_t*)bloom, (const GbMeta*)meta, entries,
+                                  ctx->d_err));
+    if ((rc = after_launch(ctx, "gd_scan_kernel"))) return rc;
+  }
+  if (b.n_rows > 0) {
+    const auto ka = pairs ? &gd_scan_all_kernel<true> : &gd_scan_all_kernel<false>;
+    const int ga = grid_res(ctx, reinterpret_cast<const void*>(ka), kGaBlock, 0, lanes);
+    const int64_t passes = pairs ? 1 : (4 * ids + kGdPassBytes - 1) / kGdPassBytes, span = (ids + passes - 1) / passes;
+    for (int64_t lo = 0; lo < ids; lo += span) {
+      BO_CUDA(ctx, launch_dependent(ka, ga, kGaBlock, 0, ctx->stream, b, c.n_rows, (int32_t)lo,
+                                    (int32_t)(std::min(lo + span, ids) - 1), (const uint8_t*)code,
+                                    (const uint32_t*)ws.cbits, (const GbMeta*)meta, filter, entries));
+      if ((rc = after_launch(ctx, "gd_scan_all_kernel"))) return rc;
+    }
+  }
+  const int wa = std::max(1, bit_length((uint64_t)prm.a_id_max));
+  const int wc = std::max(1, bit_length((uint64_t)b.n_rows));
+  const unsigned long long cmax = (wc >= 64) ? ~0ull : ((1ull << wc) - 1ull);
+  const auto kk = parts ? (pairs ? &gd_collect_kernel<true, true> : &gd_collect_kernel<true, false>)
+                        : (pairs ? &gd_collect_kernel<false, true> : &gd_collect_kernel<false, false>);
+  static bool kk_ready[2] = {false, false};
+  if (parts && !kk_ready[pairs])
+    BO_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(kk), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(4u << BO_GB_MAX_LOG2_PARTITIONS)));
+  if (parts) kk_ready[pairs] = true;
+  BO_CUDA(ctx, launch_dependent(kk, gk, kGcBlock, 4 * (size_t)n_parts, ctx->stream, (const uint32_t*)entries, ids,
+                                amask, meta, prm.year_lo, (int)prm.k, wa, cmax, part_counts, n_parts, shift, cand, out));
+  if ((rc = after_launch(ctx, "gd_collect_kernel"))) return rc;
+  if (pairs || b.n_rows == 0 || prm.k == 0) return BO_OK;
+  const void* ky = reinterpret_cast<const void*>(&gd_years_kernel);
+  BO_CUDA(ctx, launch_dependent(&gd_years_kernel, grid_res(ctx, ky, 256, 0, lanes), 256, 0, ctx->stream, b, c.n_rows,
+                                prm.year_lo, (const uint8_t*)code, out));
+  return after_launch(ctx, "gd_years_kernel");
+}
+
 int gb_finish(bo_ctx* ctx, bo_gb_result* host, const bo_gb_result* dev) {
-  BO_CUDA(ctx, cudaMemcpyAsync(host, dev, sizeof(bo_gb_result), cudaMemcpyDeviceToHost, ctx->stream));
-  uint32_t bits = 0;
-  int rc = consume_device_errors(ctx, &bits);
-  if (rc) return rc;
-  return device_error_status(ctx, bits, "groupby");
+  return read_result(ctx, "groupby", host, dev, sizeof(bo_gb_result));
 }
 
 int gb_plain_impl(bo_ctx* ctx, const bo_gb_a_cols& a, const bo_gb_b_cols& b, const bo_gb_c_cols& c,
@@ -971,6 +1736,11 @@ int bo_groupby_topk_presized_device(bo_ctx* ctx, const bo_gb_a_cols* a, const bo
   if (!pred_groups_device || !out_device) return set_error(ctx, BO_ERR_INVALID, "groupby: null prediction/output");
   GbWs ws;
   if ((rc = gb_workspace(ctx, *b, *c, prm->a_id_max, &ws))) return rc;
+  if (gb_dense_fits(*b, *prm, ws, false)) {
+    bool took = false;
+    rc = gb_dense(ctx, *a, *b, *c, *prm, ws, pred_groups_device, 0, 32, out_device, &took);
+    if (rc || took) return rc;
+  }
   if ((rc = gb_prepare(ctx, *a, *c, *prm, ws, pred_groups_device, 0))) return rc;
   return gb_aggregate_order(ctx, *b, *c, *prm, ws, out_device, 1);
 }
@@ -1004,6 +1774,12 @@ int bo_groupby_topk_partitioned_device(bo_ctx* ctx, const bo_gb_a_cols* a, const
                      BO_GB_MAX_LOG2_PARTITIONS);
   GbWs ws;
   if ((rc = gb_workspace(ctx, *b, *c, prm->a_id_max, &ws))) return rc;
+  if (gb_dense_fits(*b, *prm, ws, true)) {
+    bool took = false;
+    rc = gb_dense(ctx, *a, *b, *c, *prm, ws, nullptr, 1u << log2_partitions,
+                  log2_partitions == 0 ? 32u : (uint32_t)(32 - log2_partitions), out_device, &took);
+    if (rc || took) return rc;
+  }
   // The global group table is not used: initialise the smallest one.
   if ((rc = gb_prepare(ctx, *a, *c, *prm, ws, nullptr, kGbMinCapLog2))) return rc;
   const uint32_t n_parts = 1u << log2_partitions;

@@ -591,25 +591,6 @@ int grid_for(bo_ctx* ctx, const void* k, int block, size_t smem, int64_t work_it
   return (int)std::max<int64_t>(g, 1);
 }
 
-// Launches a kernel that may start while the previous kernel on the stream
-// still runs (programmatic dependent launch); the kernel itself waits
-// (pdl_wait) before it reads that kernel's output.
-template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*k)(KArgs...), int grid, int block, size_t smem, cudaStream_t st,
-                             Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
-}
-
 // Probe launch; a match list (eo.rows set) selects the host-gather form.
 int launch_probe(bo_ctx* ctx, const bo_join_probe_cols& p, const JoinWs& ws, bo_join_result* out, int32_t mode,
                  uint64_t probe_limit, bool dependent = false, const EmitOut& eo = EmitOut()) {
@@ -653,11 +634,7 @@ int join_run(bo_ctx* ctx, const bo_join_build_cols& b, const bo_join_probe_cols&
 }
 
 int finish_join(bo_ctx* ctx, bo_join_result* host, const bo_join_result* dev) {
-  BO_CUDA(ctx, cudaMemcpyAsync(host, dev, sizeof(bo_join_result), cudaMemcpyDeviceToHost, ctx->stream));
-  uint32_t bits = 0;
-  int rc = consume_device_errors(ctx, &bits);
-  if (rc) return rc;
-  return device_error_status(ctx, bits, "join");
+  return read_result(ctx, "join", host, dev, sizeof(bo_join_result));
 }
 
 int join_plain_impl(bo_ctx* ctx, const bo_join_build_cols& b, const bo_join_probe_cols& p, const bo_join_params& prm,

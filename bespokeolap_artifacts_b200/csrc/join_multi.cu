@@ -682,11 +682,7 @@ extern "C" int bo_join_multi_host(bo_ctx* ctx, const bo_join_build_cols* b, cons
   int rc = region(ctx, "join_multi_out", sizeof(bo_join_result) * kMq, &dout);
   if (rc) return rc;
   if ((rc = bo_join_multi_device(ctx, b, p, prm, n_queries, static_cast<bo_join_result*>(dout)))) return rc;
-  BO_CUDA(ctx, cudaMemcpyAsync(out_host, dout, sizeof(bo_join_result) * (size_t)n_queries, cudaMemcpyDeviceToHost,
-                               ctx->stream));
-  uint32_t bits = 0;
-  if ((rc = consume_device_errors(ctx, &bits))) return rc;  // synchronises the stream
-  if ((rc = device_error_status(ctx, bits, "join_multi"))) return rc;
+  if ((rc = read_result(ctx, "join_multi", out_host, dout, sizeof(bo_join_result) * (size_t)n_queries))) return rc;
   if (out_host[0].overflowed) {  // repeated build keys: every query alone, exactly
     for (int i = 0; i < n_queries; ++i) {
       if ((rc = bo_join_plain(ctx, b, p, &prm[i], &out_host[i]))) return rc;

@@ -783,10 +783,7 @@ extern "C" int bo_join_partitioned(bo_ctx* ctx, const bo_join_build_cols* b, con
   if (rc) return rc;
   if ((rc = bo_join_partitioned_device(ctx, b, p, prm, log2_partitions, static_cast<bo_join_result*>(dout))))
     return rc;
-  BO_CUDA(ctx, cudaMemcpyAsync(out_host, dout, sizeof(bo_join_result), cudaMemcpyDeviceToHost, ctx->stream));
-  uint32_t bits = 0;
-  if ((rc = consume_device_errors(ctx, &bits))) return rc;  // synchronises the stream
-  if ((rc = device_error_status(ctx, bits, "join_partitioned"))) return rc;
+  if ((rc = read_result(ctx, "join_partitioned", out_host, dout, sizeof(bo_join_result)))) return rc;
   if (out_host->overflowed) {  // a partition's table was too small: the single pass, exactly
     if ((rc = bo_join_plain(ctx, b, p, prm, out_host))) return rc;
     out_host->reruns = 1;
