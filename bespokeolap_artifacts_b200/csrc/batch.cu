@@ -21,11 +21,19 @@
 //   scan-agg  0 Q1 scan tile: per-thread shared-memory group columns, flushed
 //               into the instance's 128-bit totals; the last tile (ticket)
 //               writes the records;
-//   join      0 init (clear slots; tile 0 the Bloom filter)
-//             1 build tile (filter, CAS insert, Bloom bits)
-//             2 probe tile (Bloom filter TMA-staged in shared memory once per
-//               block and instance, warp queues, late materialisation); the
-//               last tile writes the result;
+//   join      0 init (clear slots; tile 0 the Bloom filter) and the build
+//               keys' smallest and largest value
+//             1 build tile.  Dense: where the key values in between have a bit
+//               each in the slots' memory, a qualifying key clears its bit (the
+//               empty slots are all ones); else a CAS insert and Bloom bits
+//             2 / 3 only if a dense build met a repeated key, whose
+//               multiplicity a bit cannot hold: the slots cleared again, and
+//               the hashed build after all
+//             4 probe tile.  Dense: one bit per row, read from L2; hashed: Bloom
+//               filter TMA-staged in shared memory once per block and instance,
+//               warp queues; late materialisation; the last tile writes the
+//               result.  (159M probe rows of 23 joins, whose larger builds fill
+//               the filter: BATCH_MEASURED.)
 //   group-by  0 init (slots, minima, A mask; tile 0 the Bloom filter)
 //             1 C filter tile (exact bitmap + Bloom bits) and A mask tile
 //             2 B scan tile (Bloom, exact bitmap, A mask, shared pre-aggregation
@@ -48,7 +56,7 @@ namespace {
 
 constexpr int kBB = 256;  // threads per worker block
 constexpr int kBW = kBB / 32;
-constexpr int kLevels = 4;
+constexpr int kLevels = 5;
 constexpr uint32_t kScratchBytes = 32 * 1024;
 constexpr uint32_t kSmemBytes = kBloomBytes + kScratchBytes;  // region A (Bloom / Q1 columns) + region B
 static_assert(kBB == kScanBlock, "the scan-agg columns are laid out for kScanBlock threads");
@@ -57,7 +65,10 @@ static_assert(BO_BATCH_MAX_CATS == 64, "category set size");
 enum Stage : int {
   kSQ1 = 0,
   kSJInit,
+  kSJRange,
   kSJBuild,
+  kSJReinit,
+  kSJRebuild,
   kSJProbe,
   kSGInit,
   kSGCFilter,
@@ -66,7 +77,7 @@ enum Stage : int {
   kSGSelect,
   kNumStages
 };
-constexpr int kStageLevel[kNumStages] = {0, 0, 1, 2, 0, 1, 1, 2, 3};
+constexpr int kStageLevel[kNumStages] = {0, 0, 0, 1, 2, 3, 4, 0, 1, 1, 2, 3};
 
 // Rows of one scan-agg flush period: <= 63 four-row chunks per thread plus one
 // tail row keeps every per-thread packed field inside its bits.
@@ -77,6 +88,7 @@ constexpr int64_t kQ1SubRows = (int64_t)((kMaxRowsPerThread - 1) / 4) * 4 * kBB;
 // the stage's minimum (per-item overhead) nor above the autotuned maximum.
 constexpr int64_t kTargetTiles = 2 * 148 * 2;
 constexpr int64_t kPoolMaxParticipants = 2 * 148;     // one per worker block
+constexpr int kRebuildItems = 64;
 constexpr int64_t kPoolWarps = kPoolMaxParticipants * 8;
 constexpr int64_t kPoolChunksPerWarp = 4;
 constexpr int64_t kPoolChunksPerBlock = 16;
@@ -133,11 +145,11 @@ struct InstState {
   uint32_t ticket;         // finishing ticket of the last stage
   uint32_t overflow;
   uint32_t cursor[kNumStages];  // next chunk of each pooled stage
-  uint32_t pad[1];
+  uint32_t key_max, key_nmin;   // join: largest build key and largest ~key, in unsigned order
+  uint32_t dup;                 // join: a dense build met a key twice
   // join: 0 build rows, 1 distinct keys; group-by: 0 joined, 1 distinct, 2 C passing, 3 groups
   unsigned long long cnt[4];
   unsigned long long n_cand;
-  unsigned long long pad2[3];
   unsigned long long acc[BO_Q1_MAX_GROUPS * kQ1Sums * 2];  // scan-agg 128-bit totals; join uses [0, 6)
 };
 static_assert(sizeof(InstState) % 64 == 0, "state alignment");
@@ -469,37 +481,92 @@ __device__ __forceinline__ unsigned __int128 warp_sum_u128(unsigned __int128 v) 
   return v;
 }
 
-__device__ void stage_join_init(const InstDesc& d, InstState* st, uint32_t part) {
+// Stage kSJInit, or kSJReinit (whose filter is still clear).
+__device__ void stage_join_init(const InstDesc& d, InstState* st, int stage, uint32_t part) {
   const int64_t cap = (int64_t)1 << cap_log2_of(d);
-  if (part == 0) {
+  if (part == 0 && stage == kSJInit) {
     uint4* b4 = reinterpret_cast<uint4*>(d.bloom);
     for (uint32_t i = threadIdx.x; i < kBloomWords / 4; i += kBB) b4[i] = make_uint4(0, 0, 0, 0);
   }
   ulonglong2* s2 = reinterpret_cast<ulonglong2*>(d.slots);
   const int lane = threadIdx.x & 31;
   uint32_t c;
-  while (next_chunk(&st->cursor[kSJInit], d.n_chunks[kSJInit], c)) {
+  while (next_chunk(&st->cursor[stage], d.n_chunks[stage], c)) {
     int64_t lo, hi;
-    chunk_range(c, d.unit[kSJInit], cap, lo, hi);  // even bounds: unit and cap are even
+    chunk_range(c, d.unit[stage], cap, lo, hi);  // even bounds: unit and cap are even
     for (int64_t i = lo / 2 + lane; i < hi / 2; i += 32) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
   }
 }
 
-__device__ void stage_join_build(const InstDesc& d, InstState* st, const Smem& sm, uint32_t (*red)[kBW]) {
+constexpr uint32_t kKeySign = 0x80000000u;  // int32 order as uint32 order
+
+__device__ void stage_join_range(const InstDesc& d, InstState* st) {
+  const int32_t* key = d.build.key;
+  const int lane = threadIdx.x & 31;
+  uint32_t kmax = 0, nmin = 0, c;
+  auto take = [&](int32_t v) {
+    const uint32_t k = (uint32_t)v ^ kKeySign;
+    kmax = max(kmax, k);
+    nmin = max(nmin, ~k);
+  };
+  while (next_chunk(&st->cursor[kSJRange], d.n_chunks[kSJRange], c)) {
+    int64_t lo, hi;
+    chunk_range(c, d.unit[kSJRange], d.build.n_rows, lo, hi);
+    for (int64_t r = lo + lane * 8; r < hi; r += 256) {
+      if (r + 8 <= hi) {
+        const int8v k = ld_stream_v8(key + r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) take(k.v[j]);
+      } else {
+        for (int64_t i = r; i < hi; ++i) take(key[i]);
+      }
+    }
+  }
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  nmin = __reduce_max_sync(0xffffffffu, nmin);
+  if (lane == 0 && (kmax | nmin)) {
+    atomicMax(&st->key_max, kmax);
+    atomicMax(&st->key_nmin, nmin);
+  }
+}
+
+// After level 0: whether the join keeps one bit per key value, from `base` on.
+struct JoinDense {
+  bool on;
+  uint32_t base, range;
+};
+
+__device__ __forceinline__ JoinDense join_dense(const InstDesc& d, const InstState* st, int32_t cap_log2) {
+  const uint32_t lo = ~__ldcg(&st->key_nmin), hi = __ldcg(&st->key_max);
+  const uint64_t range = (uint64_t)hi - lo + 1;
+  JoinDense j;
+  j.on = d.build.n_rows > 0 && range <= min(64ull << cap_log2, 0xffffffffull);
+  j.base = lo ^ kKeySign;
+  j.range = (uint32_t)range;
+  return j;
+}
+
+// Stage kSJBuild, or kSJRebuild (hashed, everything but the table counted
+// already).
+__device__ void stage_join_build(const InstDesc& d, InstState* st, int stage, const Smem& sm, uint32_t (*red)[kBW]) {
   const bo_join_build_cols b = d.build;
   const int32_t date_lt = d.date_lt;
   const uint32_t seg = d.seg;
   unsigned long long* slots = d.slots;
   uint32_t* bloom = d.bloom;
-  const uint64_t mask = (1ull << cap_log2_of(d)) - 1;
+  const int32_t cl = cap_log2_of(d);
+  const uint64_t mask = (1ull << cl) - 1;
+  JoinDense dense = join_dense(d, st, cl);
+  if (stage == kSJRebuild) dense.on = false;
+  uint32_t* bits = reinterpret_cast<uint32_t*>(d.slots);
   const int lane = threadIdx.x & 31;
   uint32_t* bq = reinterpret_cast<uint32_t*>(sm.b) + (threadIdx.x >> 5) * 256;
-  uint32_t qual = 0, newkeys = 0;
+  uint32_t qual = 0, newkeys = 0, dup = 0;
   bool full = false;
   uint32_t c;
-  while (next_chunk(&st->cursor[kSJBuild], d.n_chunks[kSJBuild], c)) {
+  while (next_chunk(&st->cursor[stage], d.n_chunks[stage], c)) {
     int64_t lo, hi;
-    chunk_range(c, d.unit[kSJBuild], b.n_rows, lo, hi);
+    chunk_range(c, d.unit[stage], b.n_rows, lo, hi);
     for (int64_t base = lo; base < hi; base += 512) {  // warp-uniform: 16 rows per lane
       const int64_t r0 = base + lane * 16;
       uint32_t q = 0;
@@ -527,15 +594,25 @@ __device__ void stage_join_build(const InstDesc& d, InstState* st, const Smem& s
         for (int k = 0; k < 8; ++k)
           if ((hm >> k) & 1u) bq[pos++] = (uint32_t)(lane * 16 + 8 * half + k);
         __syncwarp();
-        for (uint32_t i = lane; i < total; i += 32)
-          join_insert(slots, bloom, mask, __ldg(b.key + base + bq[i]), newkeys, full, kPresizedProbeLimit);
+        for (uint32_t i = lane; i < total; i += 32) {
+          const int32_t key = __ldg(b.key + base + bq[i]);
+          if (dense.on) {
+            const uint32_t off = (uint32_t)key - dense.base, bit = 1u << (off & 31u);
+            if (atomicAnd(bits + (off >> 5), ~bit) & bit) ++newkeys;
+            else dup = 1;
+          } else {
+            join_insert(slots, bloom, mask, key, newkeys, full, kPresizedProbeLimit);
+          }
+        }
         __syncwarp();
       }
     }
   }
   uint32_t tot[4];
-  block_counts(qual, newkeys, 0, full, red, tot);
+  block_counts(qual, newkeys, dup, full, red, tot);
   if (threadIdx.x == 0) {
+    if (tot[2]) atomicOr(&st->dup, 1u);
+    if (stage == kSJRebuild) tot[0] = tot[1] = 0;
     if (tot[0]) atomicAdd(&st->cnt[0], (unsigned long long)tot[0]);
     if (tot[1]) {
       const unsigned long long before = atomicAdd(&st->cnt[1], (unsigned long long)tot[1]);
@@ -545,8 +622,33 @@ __device__ void stage_join_build(const InstDesc& d, InstState* st, const Smem& s
   }
 }
 
+// Dense probe of rows [lo, hi) by one warp, lane-strided so that the price /
+// discount loads of matching rows coalesce.
+__device__ __forceinline__ void probe_dense(const bo_join_probe_cols& p, const uint32_t* bits, const JoinDense& dense,
+                                            int64_t lo, int64_t hi, ProbeAcc& acc) {
+  constexpr int kRows = 8;
+  for (int64_t base = lo + (threadIdx.x & 31); base - (threadIdx.x & 31) < hi; base += 32 * kRows) {
+    uint32_t off[kRows], word[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      off[j] = base + 32 * j < hi ? (uint32_t)__ldcs(p.fk + base + 32 * j) - dense.base : 0xffffffffu;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) word[j] = off[j] < dense.range ? __ldcg(bits + (off[j] >> 5)) : 0xffffffffu;
+    uint64_t pr[kRows], dc[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      const bool hit = !((word[j] >> (off[j] & 31u)) & 1u);
+      pr[j] = hit ? (uint64_t)__ldcs(p.price + base + 32 * j) : 0u;
+      dc[j] = hit ? (uint64_t)__ldcs(p.discount + base + 32 * j) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      if (!((word[j] >> (off[j] & 31u)) & 1u)) accumulate_match(pr[j], dc[j], 1ull, acc);
+  }
+}
+
 __device__ void stage_join_probe(const InstDesc& d, InstState* st, const Smem& sm, const uint32_t* bl, uint32_t wmask,
-                                 bo_batch_result* res, uint32_t* flag, uint32_t* err) {
+                                 const JoinDense& dense, bo_batch_result* res, uint32_t* flag, uint32_t* err) {
   const bo_join_probe_cols p = d.probe;
   const int32_t cl = cap_log2_of(d);
   const uint64_t mask = (1ull << cl) - 1;
@@ -560,6 +662,10 @@ __device__ void stage_join_probe(const InstDesc& d, InstState* st, const Smem& s
   while (next_chunk(&st->cursor[kSJProbe], d.n_chunks[kSJProbe], c)) {
     int64_t lo, hi;
     chunk_range(c, d.unit[kSJProbe], p.n_rows, lo, hi);
+    if (dense.on) {
+      probe_dense(p, reinterpret_cast<const uint32_t*>(slots), dense, lo, hi, acc);
+      continue;
+    }
     for (int64_t base = lo; base < hi; base += 512) {
       const int64_t r0 = base + lane * 16;
       int32_t fk[16];
@@ -1089,7 +1195,19 @@ __global__ void __launch_bounds__(kBB, 2)
     // Stages that read a Bloom filter stage it into region A once per block and instance.
     const uint32_t* bl = reinterpret_cast<const uint32_t*>(sm.a);
     uint32_t wmask = kBloomWords - 1u;
-    if (stage == kSJProbe || stage == kSGScan) {
+    JoinDense dense{false, 0u, 0u};
+    if (stage >= kSJBuild && stage <= kSJProbe) {
+      dense = join_dense(d, st, cap_log2_of(d));
+      const bool again = dense.on && __ldcg(&st->dup);  // the hashed build replaces the dense one
+      if ((stage == kSJReinit || stage == kSJRebuild) && !again) {
+        __threadfence();
+        if (threadIdx.x == 0) atomicAdd(&st->done[level], 1u);
+        __syncthreads();  // `cur` has been read by every thread
+        continue;
+      }
+      if (stage == kSJProbe && again) dense.on = false;
+    }
+    if ((stage == kSJProbe && !dense.on) || stage == kSGScan) {
       if (bloom_inst != (int32_t)inst) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -1122,13 +1240,18 @@ __global__ void __launch_bounds__(kBB, 2)
         stage_q1(d, st, tile, sm, res, &flag, err);
         break;
       case kSJInit:
-        stage_join_init(d, st, tile);
+      case kSJReinit:
+        stage_join_init(d, st, (int)stage, tile);
+        break;
+      case kSJRange:
+        stage_join_range(d, st);
         break;
       case kSJBuild:
-        stage_join_build(d, st, sm, red);
+      case kSJRebuild:
+        stage_join_build(d, st, (int)stage, sm, red);
         break;
       case kSJProbe:
-        stage_join_probe(d, st, sm, bl, wmask, res, &flag, err);
+        stage_join_probe(d, st, sm, bl, wmask, dense, res, &flag, err);
         break;
       case kSGInit:
         stage_gb_init(d, st, tile);
@@ -1307,6 +1430,11 @@ int check_instance(bo_ctx* ctx, const bo_batch_instance& x, int i) {
 
 size_t al256(size_t v) { return (v + 255) & ~size_t(255); }
 
+// Items of the join's key range and second build are not counted against a
+// caller's item limit: every plan has room for them beside it.
+bool own_items(int stage) { return stage == kSJRange || stage == kSJReinit || stage == kSJRebuild; }
+constexpr int64_t kOwnItems = kPoolMaxParticipants + 2 * kRebuildItems;  // per instance, at most
+
 struct Plan {
   InstDesc d;
   size_t table_bytes;
@@ -1346,7 +1474,12 @@ Plan plan_instance(const bo_batch_instance& x) {
     d.cap_log2 = x.predicted_device ? max_log2 : presize(x.predicted, factor, max_log2);
     const int64_t cap = (int64_t)1 << d.cap_log2;
     pool_stage(d, kSJInit, cap, 2048, 1 << 16, 2048);
+    pool_stage(d, kSJRange, x.build.n_rows, 2048, 2 * t, 256);
     pool_stage(d, kSJBuild, x.build.n_rows, 512, 2 * t, 512);
+    // The second build is rare: fewer items to pass over when it is not needed.
+    pool_stage(d, kSJReinit, cap, 2048, 1 << 16, 2048);
+    pool_stage(d, kSJRebuild, x.build.n_rows, 512, 2 * t, 512);
+    for (int s : {kSJReinit, kSJRebuild}) d.n_tiles[s] = std::min(d.n_tiles[s], (uint32_t)kRebuildItems);
     pool_stage(d, kSJProbe, x.probe.n_rows, 512, t, 512);
     p.table_bytes = al256(8 * (size_t)cap) + al256(kBloomBytes);
     p.weight = 9.0 * (double)x.build.n_rows + 20.0 * (double)x.probe.n_rows;
@@ -1386,7 +1519,7 @@ Plan plan_instance(const bo_batch_instance& x) {
   p.items = 0;
   for (int s = 0; s < kNumStages; ++s) {
     if (d.n_tiles[s]) d.level_items[kStageLevel[s]] += d.n_tiles[s];
-    p.items += d.n_tiles[s];
+    if (!own_items(s)) p.items += d.n_tiles[s];
   }
   return p;
 }
@@ -1487,7 +1620,8 @@ int create_batch(bo_ctx* ctx, int32_t max_instances, int64_t max_items, size_t p
   b->max_instances = max_instances;
   b->max_items = max_items;
   b->pool_bytes = pool_bytes;
-  b->plan_bytes = kPlanHdr + al256(sizeof(InstDesc) * max_instances) + al256(sizeof(uint2) * (size_t)max_items);
+  b->plan_bytes = kPlanHdr + al256(sizeof(InstDesc) * max_instances) +
+                  al256(sizeof(uint2) * (size_t)(max_items + kOwnItems * max_instances));
   b->state_bytes = 256 + sizeof(InstState) * max_instances;
   const size_t off_ctl = al256(b->plan_bytes);
   const size_t off_res = off_ctl + al256(b->state_bytes);
