@@ -34,6 +34,7 @@
 #include "common.cuh"
 #include "compact.cuh"
 #include "context.cuh"
+#include "small_sort.cuh"
 
 namespace bo {
 namespace {
@@ -44,30 +45,6 @@ constexpr int kQ18RowsPerThread = 8;
 int grid_for(bo_ctx* ctx, int64_t items) {
   const int64_t need = (items + kTpBlock - 1) / kTpBlock;
   return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)ctx->num_sms * 8));
-}
-
-// Block-level compaction step: every thread of the block calls it with its
-// keep flag; the block reserves its total once.  Returns the output position
-// of a kept element.
-__device__ __forceinline__ unsigned long long block_reserve(bool keep, unsigned long long* n_out,
-                                                            uint32_t* warp_off, unsigned long long* base) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t m = __ballot_sync(0xffffffffu, keep);
-  if (lane == 0) warp_off[warp] = __popc(m);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t t = 0;
-    for (int w = 0; w < kTpBlock / 32; ++w) {
-      const uint32_t c = warp_off[w];
-      warp_off[w] = t;
-      t += c;
-    }
-    *base = t ? atomicAdd(n_out, (unsigned long long)t) : 0ull;
-  }
-  __syncthreads();
-  const unsigned long long pos = *base + warp_off[warp] + __popc(m & ((1u << lane) - 1u));
-  __syncthreads();  // warp_off / base are rewritten by the next call
-  return pos;
 }
 
 // ------------------------------------------------------------ order ranges --
@@ -269,6 +246,7 @@ __device__ __forceinline__ void q18_add(Q18Run& run, int32_t key, int16_t q, int
 __global__ void q18_sum_kernel(const int32_t* __restrict__ l_orderkey, const int16_t* __restrict__ l_quantity,
                                int64_t n, int64_t bound, int dense, uint32_t* __restrict__ sum,
                                uint32_t* __restrict__ mark, uint32_t* err) {
+  pdl_launch_dependents();
   const int64_t groups = n / kQ18RowsPerThread;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -314,7 +292,15 @@ struct Q18Cust {
   }
 };
 
-// (orderkey, orders row) of every qualifying order.
+// (orderkey, orders row) of every qualifying order, in no particular order: a
+// block lists its own and reserves their places when the list might not take
+// another step's, and at the end.  Four rows per thread and step, whose sums
+// are requested together: the sums are random reads, and one row at a time the
+// pass waited on them (18 us for 1.5M orders, now 15; eight rows at once: 27).
+constexpr int kQ18Orders = 4;
+constexpr int kQ18Step = kTpBlock * kQ18Orders;
+constexpr int kQ18List = 2 * kQ18Step;
+
 __global__ void __launch_bounds__(kTpBlock) q18_qualify_kernel(const int32_t* __restrict__ o_orderkey,
                                                                const int32_t* __restrict__ o_custkey,
                                                                int64_t n_orders, int dense, int64_t bound,
@@ -324,29 +310,75 @@ __global__ void __launch_bounds__(kTpBlock) q18_qualify_kernel(const int32_t* __
                                                                unsigned long long* __restrict__ keys,
                                                                uint32_t* __restrict__ vals,
                                                                unsigned long long* n_out, uint32_t* err) {
-  __shared__ uint32_t warp_off[kTpBlock / 32];
+  __shared__ uint2 mine[kQ18List];
+  __shared__ uint32_t n_mine;
   __shared__ unsigned long long base;
-  for (int64_t b0 = (int64_t)blockIdx.x * kTpBlock; b0 < n_orders; b0 += (int64_t)gridDim.x * kTpBlock) {
-    const int64_t row = b0 + threadIdx.x;
-    bool keep = false;
-    int32_t key = 0;
-    if (row < n_orders) {
-      key = dense ? (int32_t)(row + 1) : o_orderkey[row];
-      if (key < 0 || (int64_t)key >= bound) {
-        raise_error(err, kErrValueRange);
-      } else if (sum[key] > threshold && (!mark || ((mark[key >> 5] >> (key & 31)) & 1u))) {
-        keep = cust.row_of(o_custkey[row]) >= 0;
+  if (threadIdx.x == 0) n_mine = 0;
+  __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();
+  auto flush = [&]() {  // all threads; n_mine is settled
+    const uint32_t n = n_mine;
+    if (threadIdx.x == 0) base = n ? atomicAdd(n_out, (unsigned long long)n) : 0ull;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += kTpBlock) {
+      keys[base + i] = mine[i].x;
+      vals[base + i] = mine[i].y;
+    }
+    if (threadIdx.x == 0) n_mine = 0;
+    __syncthreads();
+  };
+  for (int64_t b0 = (int64_t)blockIdx.x * kQ18Step; b0 < n_orders; b0 += (int64_t)gridDim.x * kQ18Step) {
+    int32_t key[kQ18Orders], qty[kQ18Orders];
+    uint32_t ok = 0;
+#pragma unroll
+    for (int j = 0; j < kQ18Orders; ++j) {
+      const int64_t row = b0 + j * kTpBlock + threadIdx.x;
+      key[j] = row < n_orders ? (dense ? (int32_t)(row + 1) : o_orderkey[row]) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < kQ18Orders; ++j) {
+      const bool in = key[j] >= 0 && (int64_t)key[j] < bound;
+      if (b0 + j * kTpBlock + threadIdx.x < n_orders) {
+        if (in) ok |= 1u << j;
+        else raise_error(err, kErrValueRange);
       }
+      qty[j] = in ? __ldg(sum + key[j]) : 0;
     }
-    const unsigned long long pos = block_reserve(keep, n_out, warp_off, &base);
-    if (keep) {
-      keys[pos] = (unsigned long long)((uint32_t)key ^ 0x80000000u);
-      vals[pos] = (uint32_t)row;
+#pragma unroll
+    for (int j = 0; j < kQ18Orders; ++j) {
+      const int64_t row = b0 + j * kTpBlock + threadIdx.x;
+      if (!((ok >> j) & 1u) || qty[j] <= threshold) continue;
+      if (mark && !((mark[key[j] >> 5] >> (key[j] & 31)) & 1u)) continue;
+      if (cust.row_of(o_custkey[row]) < 0) continue;
+      mine[atomicAdd(&n_mine, 1u)] = make_uint2((uint32_t)key[j] ^ 0x80000000u, (uint32_t)row);
     }
+    __syncthreads();
+    const bool full = n_mine > (uint32_t)(kQ18List - kQ18Step);
+    __syncthreads();  // the next step adds to n_mine
+    if (full) flush();
   }
+  flush();
 }
 
 // (totalprice desc, orderdate asc) as one 48-bit ascending key.
+__device__ __forceinline__ unsigned long long q18_sort_key(int32_t price, int16_t date) {
+  const uint32_t price_desc = ~((uint32_t)price ^ 0x80000000u);
+  return ((unsigned long long)price_desc << 16) | ((uint32_t)(uint16_t)date ^ 0x8000u);
+}
+
+// Qualifying order i as an item of the small sort (ties by orderkey).
+struct Q18Item {
+  const unsigned long long* keys;
+  const uint32_t* vals;
+  const int32_t* o_totalprice;
+  const int16_t* o_orderdate;
+  __device__ __forceinline__ uint4 operator()(uint32_t i) const {
+    const uint32_t row = vals[i];
+    return ss_item(q18_sort_key(o_totalprice[row], o_orderdate[row]), (uint32_t)keys[i], row);
+  }
+};
+
 __global__ void q18_key2_kernel(const uint32_t* __restrict__ vals, const int32_t* __restrict__ o_totalprice,
                                 const int16_t* __restrict__ o_orderdate, const unsigned long long* n_out,
                                 unsigned long long* __restrict__ keys) {
@@ -354,9 +386,7 @@ __global__ void q18_key2_kernel(const uint32_t* __restrict__ vals, const int32_t
   for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (unsigned long long)gridDim.x * blockDim.x) {
     const uint32_t row = vals[i];
-    const uint32_t price_desc = ~((uint32_t)o_totalprice[row] ^ 0x80000000u);
-    const uint32_t date_asc = (uint32_t)(uint16_t)o_orderdate[row] ^ 0x8000u;
-    keys[i] = ((unsigned long long)price_desc << 16) | date_asc;
+    keys[i] = q18_sort_key(o_totalprice[row], o_orderdate[row]);
   }
 }
 
@@ -369,8 +399,13 @@ __global__ void __launch_bounds__(kQ18RowsBlock) q18_gather_kernel(
     const uint32_t* __restrict__ vals, const int32_t* __restrict__ o_orderkey, const int32_t* __restrict__ o_custkey,
     const int16_t* __restrict__ o_orderdate, const int32_t* __restrict__ o_totalprice, int dense,
     const int32_t* __restrict__ sum, Q18Cust cust, const unsigned long long* n_out, unsigned long long limit,
-    bo_tpch_q18_row* __restrict__ out) {
+    bo_tpch_q18_row* __restrict__ out, HostWords words) {
   __shared__ bo_tpch_q18_row stage[kQ18RowsBlock];
+  pdl_wait();
+  if (words.words) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) words.store();
+    if (*words.overflow) return;  // vals were not sorted
+  }
   constexpr int kWords = (int)(sizeof(bo_tpch_q18_row) / 16);
   static_assert(sizeof(bo_tpch_q18_row) % 16 == 0, "rows are whole 16-byte words");
   const unsigned long long n = *n_out < limit ? *n_out : limit;  // the first min(count, limit) rows
@@ -658,13 +693,12 @@ extern "C" int bo_tpch_q10_host_rows(bo_ctx* ctx, const bo_tpch_q10_tables* t, i
 }
 
 namespace {
-// counted: both sorts read the result count on the device and the rows go
-// straight into out_host where it is mapped pinned memory (one
-// synchronisation); a count beyond one cluster sort reruns the whole query
-// with the count read back before the sorts (the second sort's keys replace
-// the first's, so the rerun starts over).
+// The sort reads the result count on the device and the rows go straight into
+// out_host where it is mapped pinned memory (one synchronisation); a count
+// beyond the small sort goes on, once it was read back, with two stable sorts
+// of the listed orders.
 int q18_run(bo_ctx* ctx, const bo_tpch_q18_tables* t, int32_t quantity_threshold, bo_tpch_q18_row* out_host,
-            int64_t max_rows, int64_t* n_rows, bool counted) {
+            int64_t max_rows, int64_t* n_rows) {
   if (!t || !n_rows || max_rows < 0 || (max_rows > 0 && !out_host))
     return set_error(ctx, BO_ERR_INVALID, "q18: null argument");
   if (t->n_orders < 0 || t->n_lineitem < 0 || t->n_custkey_map < 0 || t->n_customer < 0 || t->orderkey_bound < 0)
@@ -689,29 +723,32 @@ int q18_run(bo_ctx* ctx, const bo_tpch_q18_tables* t, int32_t quantity_threshold
   const int64_t cap = std::max<int64_t>(no, 1);
   size_t total = 0;
   auto add = [&](size_t b) { total += (b + 255) & ~size_t(255); };
+  add(64);
   add(4 * (size_t)bound);
   add(4 * (size_t)std::max<int64_t>(mark_words, 1));
+  add(kSsItemBytes);
+  add(4 * (size_t)kSmallSortMax);
   add(8 * (size_t)cap);
   add(4 * (size_t)cap);
   add(8 * (size_t)cap);
   add(4 * (size_t)cap);
   add(sizeof(bo_tpch_q18_row) * (size_t)cap);
-  add(64);
   void* basep = nullptr;
   int rc = region(ctx, "q18_ws", total, &basep);
   if (rc) return rc;
   char* p = static_cast<char*>(basep);
+  auto* n_out = carve<unsigned long long>(p, 8);
   auto* sum = carve<int32_t>(p, (size_t)bound);
   auto* mark = carve<uint32_t>(p, (size_t)std::max<int64_t>(mark_words, 1));
+  const size_t zeroed = (size_t)(p - static_cast<char*>(basep));
+  auto* items = carve<char>(p, kSsItemBytes);
+  auto* sorted = carve<uint32_t>(p, (size_t)kSmallSortMax);
   auto* keys = carve<unsigned long long>(p, (size_t)cap);
   auto* vals = carve<uint32_t>(p, (size_t)cap);
   auto* tkeys = carve<unsigned long long>(p, (size_t)cap);
   auto* tvals = carve<uint32_t>(p, (size_t)cap);
   auto* rows = carve<bo_tpch_q18_row>(p, (size_t)cap);
-  auto* n_out = carve<unsigned long long>(p, 8);
-  BO_CUDA(ctx, cudaMemsetAsync(sum, 0, 4 * (size_t)bound, ctx->stream));
-  if (use_mark) BO_CUDA(ctx, cudaMemsetAsync(mark, 0, 4 * (size_t)mark_words, ctx->stream));
-  BO_CUDA(ctx, cudaMemsetAsync(n_out, 0, 16, ctx->stream));  // the count and the sorts' overflow word
+  BO_CUDA(ctx, cudaMemsetAsync(basep, 0, zeroed, ctx->stream));  // the count, the overflow word, sums and marks
   if (t->n_lineitem > 0) {
     const int64_t threads = t->n_lineitem / kQ18RowsPerThread + kQ18RowsPerThread;
     q18_sum_kernel<<<grid_for(ctx, threads), kTpBlock, 0, ctx->stream>>>(
@@ -721,49 +758,46 @@ int q18_run(bo_ctx* ctx, const bo_tpch_q18_tables* t, int32_t quantity_threshold
   }
   if (no == 0) return finish_rows(ctx, "q18", n_out, rows, out_host, max_rows, n_rows);
   const Q18Cust cust{t->custkey_to_row, t->n_custkey_map, t->n_customer, dense && t->dense_custkeys != 0};
-  q18_qualify_kernel<<<grid_for(ctx, no), kTpBlock, 0, ctx->stream>>>(
-      t->o_orderkey, t->o_custkey, no, dense ? 1 : 0, bound, sum, use_mark ? mark : nullptr, quantity_threshold,
-      cust, keys, vals, n_out, ctx->d_err);
+  BO_CUDA(ctx, launch_dependent(&q18_qualify_kernel, grid_for(ctx, (no + kQ18Orders - 1) / kQ18Orders), kTpBlock, 0,
+                                ctx->stream, t->o_orderkey, t->o_custkey, no, dense ? 1 : 0, bound,
+                                (const int32_t*)sum, (const uint32_t*)(use_mark ? mark : nullptr), quantity_threshold,
+                                cust, keys, vals, n_out, ctx->d_err));
   if ((rc = after_launch(ctx, "q18_qualify_kernel"))) return rc;
   uint32_t* overflow = reinterpret_cast<uint32_t*>(n_out + 1);
+  if ((rc = small_sort(ctx, Q18Item{keys, vals, t->o_totalprice, t->o_orderdate}, n_out, items, sorted, overflow)))
+    return rc;
+  bo_tpch_q18_row* direct = max_rows > 0 ? static_cast<bo_tpch_q18_row*>(mapped_device_ptr(out_host)) : nullptr;
+  auto gather = [&](const uint32_t* order, HostWords words) -> int {
+    const int64_t lim = direct ? std::min<int64_t>(max_rows, cap) : cap;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((lim + kQ18RowsBlock - 1) / kQ18RowsBlock,
+                                                                 (int64_t)ctx->num_sms * 8));
+    BO_CUDA(ctx, launch_dependent(&q18_gather_kernel, grid, kQ18RowsBlock, 0, ctx->stream, order, t->o_orderkey,
+                                  t->o_custkey, t->o_orderdate, t->o_totalprice, dense ? 1 : 0, (const int32_t*)sum,
+                                  cust, (const unsigned long long*)n_out, (unsigned long long)lim,
+                                  direct ? direct : rows, words));
+    return after_launch(ctx, "q18_gather_kernel");
+  };
+  if ((rc = gather(sorted, HostWords{ctx->h_word, n_out, overflow, ctx->d_err}))) return rc;
   int64_t ns = 0;
-  if (!counted) {  // the result's size, read back once before the sorts
-    if ((rc = read_device_count(ctx, n_out, cap, &ns))) return rc;
-    if ((rc = radix_sort_pairs(ctx, keys, vals, tkeys, tvals, ns, 0, 32, nullptr))) return rc;
-  } else if ((rc = cluster_sort_pairs_counted(ctx, keys, vals, n_out, cap, 0, 32, overflow))) {
-    return rc;
-  }
-  q18_key2_kernel<<<grid_for(ctx, no), kTpBlock, 0, ctx->stream>>>(vals, t->o_totalprice, t->o_orderdate, n_out,
-                                                                     keys);
-  if ((rc = after_launch(ctx, "q18_key2_kernel"))) return rc;
-  if (!counted) {
-    if ((rc = radix_sort_pairs(ctx, keys, vals, tkeys, tvals, ns, 0, 48, nullptr))) return rc;
-  } else if ((rc = cluster_sort_pairs_counted(ctx, keys, vals, n_out, cap, 0, 48, overflow))) {
-    return rc;
-  }
-  bo_tpch_q18_row* direct =
-      (counted && max_rows > 0) ? static_cast<bo_tpch_q18_row*>(mapped_device_ptr(out_host)) : nullptr;
-  const int64_t lim = direct ? std::min<int64_t>(max_rows, cap) : cap;
-  const int ggrid = (int)std::max<int64_t>(1, std::min<int64_t>((lim + kQ18RowsBlock - 1) / kQ18RowsBlock,
-                                                                  (int64_t)ctx->num_sms * 8));
-  q18_gather_kernel<<<ggrid, kQ18RowsBlock, 0, ctx->stream>>>(vals, t->o_orderkey, t->o_custkey, t->o_orderdate,
-                                                              t->o_totalprice, dense ? 1 : 0, sum, cust, n_out,
-                                                              (unsigned long long)lim, direct ? direct : rows);
-  if ((rc = after_launch(ctx, "q18_gather_kernel"))) return rc;
-  if (!counted) return finish_known_rows(ctx, "q18", ns, rows, out_host, max_rows, n_rows);
   bool over = false;
-  if ((rc = read_counted(ctx, "q18", n_out, cap, &ns, &over))) return rc;
-  if (over) return q18_run(ctx, t, quantity_threshold, out_host, max_rows, n_rows, false);
-  if (direct) {
+  if ((rc = read_host_words(ctx, "q18", cap, &ns, &over))) return rc;
+  if (over) {  // by orderkey, then stably by (totalprice desc, orderdate asc)
+    if ((rc = radix_sort_pairs(ctx, keys, vals, tkeys, tvals, ns, 0, 32, nullptr))) return rc;
+    q18_key2_kernel<<<grid_for(ctx, ns), kTpBlock, 0, ctx->stream>>>(vals, t->o_totalprice, t->o_orderdate, n_out,
+                                                                       keys);
+    if ((rc = after_launch(ctx, "q18_key2_kernel"))) return rc;
+    if ((rc = radix_sort_pairs(ctx, keys, vals, tkeys, tvals, ns, 0, 48, nullptr))) return rc;
+    if ((rc = gather(vals, HostWords{}))) return rc;
+  } else if (direct) {
     *n_rows = ns;
     return BO_OK;
   }
-  return finish_known_rows(ctx, "q18", ns, rows, out_host, max_rows, n_rows);
+  return finish_known_rows(ctx, "q18", ns, rows, out_host, direct ? 0 : max_rows, n_rows);
 }
 }  // namespace
 
 extern "C" int bo_tpch_q18(bo_ctx* ctx, const bo_tpch_q18_tables* t, int32_t quantity_threshold,
                            bo_tpch_q18_row* out_host, int64_t max_rows, int64_t* n_rows) {
   BO_CHECK_CTX(ctx);
-  return q18_run(ctx, t, quantity_threshold, out_host, max_rows, n_rows, true);
+  return q18_run(ctx, t, quantity_threshold, out_host, max_rows, n_rows);
 }
