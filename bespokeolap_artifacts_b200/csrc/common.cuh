@@ -182,25 +182,27 @@ __host__ __device__ __forceinline__ bo_i128 to_bo_i128(__int128 v) {
   return r;
 }
 
-// Sum of an unsigned 128-bit value over the block, returned in thread 0.
-// `scratch` holds blockDim.x + 32 entries.  Warp leaders add their warp's
-// values serially in 128 bits, thread 0 adds the warp totals: exact for any
-// inputs, and cheap because it runs once per block.
-__device__ __forceinline__ unsigned __int128 block_sum_u128(unsigned __int128 v, unsigned __int128* scratch) {
-  scratch[threadIdx.x] = v;
-  __syncthreads();
-  const int nw = (int)(blockDim.x >> 5);
-  if ((threadIdx.x & 31) == 0) {
-    unsigned __int128 t = 0;
-    for (int i = 0; i < 32; ++i) t += scratch[threadIdx.x + i];
-    scratch[blockDim.x + (threadIdx.x >> 5)] = t;
+// Sum of an unsigned 128-bit value over the block, returned in thread 0 (0 in
+// the others).  `scratch` holds an entry per warp.
+__device__ __forceinline__ unsigned __int128 warp_sum_u128(unsigned __int128 v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long lo = __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
+    const unsigned long long hi = __shfl_xor_sync(0xffffffffu, (unsigned long long)(v >> 64), o);
+    v += ((unsigned __int128)hi << 64) | lo;
   }
+  return v;
+}
+
+__device__ __forceinline__ unsigned __int128 block_sum_u128(unsigned __int128 v, unsigned __int128* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  v = warp_sum_u128(v);
+  if (lane == 0) scratch[warp] = v;
   __syncthreads();
   unsigned __int128 tot = 0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < nw; ++w) tot += scratch[blockDim.x + w];
+  if (warp == 0) tot = warp_sum_u128(lane < nw ? scratch[lane] : (unsigned __int128)0);
   __syncthreads();
-  return tot;
+  return threadIdx.x == 0 ? tot : (unsigned __int128)0;
 }
 
 // Last-block epilogue: true in every thread of the block that finished last

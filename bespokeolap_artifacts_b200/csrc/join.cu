@@ -11,7 +11,9 @@
 //   build  (K2)                    filter build rows, insert keys with 64-bit
 //                                  atomicCAS into open-addressing slots
 //                                  (key << 32 | multiplicity), set 2 bits of a
-//                                  blocked Bloom filter per new key;
+//                                  blocked Bloom filter per new key; keys in
+//                                  range set a bit of their own besides, or,
+//                                  where very many are expected, instead;
 //   probe  (K3)                    each block stages the 64 KB Bloom filter into
 //                                  shared memory with one TMA bulk copy; probe
 //                                  rows stream in 8 per lane (one 256-bit fk
@@ -19,7 +21,10 @@
 //                                  table; only matching rows load their price and
 //                                  discount (late materialisation); exact
 //                                  fixed-point sums, 128-bit totals, last block
-//                                  writes the result.
+//                                  writes the result.  Key bits take the
+//                                  filter's place in shared memory where all
+//                                  fit (kSmemBits), or the table's in L2
+//                                  (kBitsCapLog2).
 // Build-side keys are read densely with the filter columns (one streaming pass).
 #include <algorithm>
 #include <string>
@@ -45,11 +50,32 @@ constexpr int kMinCapLog2 = 10;
 constexpr float kPresizeFactor = 4.0f;
 constexpr uint64_t kPlainSlotsPerRow = 4;
 
+// From this capacity on (524 thousand expected keys and more) build keys within
+// [0, kBitsPerRow * build rows) are one bit each and only the others, and the
+// repeats of a key, are hashed: the 64 KB Bloom filter passes most rows by then
+// and each costs a random read of a table that outgrows L2, where one L2 read
+// of a bit answers every row.  Hashed against bits, 20M probe rows: 200
+// thousand keys 119 / 142 us, 800 thousand 311 / 176; 60M: 200 thousand keys 263
+// / 354, 600 thousand 512 / 386, 3 million 1360 / 473.
+constexpr int kBitsCapLog2 = 22;
+constexpr int64_t kBitsPerRow = 16;
+
+// Build sides of at most this many rows: keys are hashed, and those within [0,
+// 4 x build rows), at most this many, are bits besides, which the probe keeps in
+// shared memory instead of the Bloom filter (192 KB, what one block per SM has
+// beside its queues).  They answer every row, so matches need no look at the
+// table; a key without a bit, or a repeated one, leaves the probe to the filter
+// and the table.  Filter against bits: 250 thousand x 1M rows 26.6 / 23.5 us, 1.5M
+// x 6M with 60 / 120 / 300 thousand keys 39 / 35, 50 / 41 and 77 / 57 us.
+constexpr int64_t kSmemBits = 1536000;
+
 // Device-resident join state (one per context, in the "join_meta" region).
 struct JoinMeta {
   int32_t cap_log2;
   uint32_t done;               // probe ticket counter
   uint32_t overflow;           // presized table too small
+  uint32_t n_bits;             // keys kept as one bit each: [0, n_bits), 0 if all are hashed
+  uint32_t hashed;             // the bits alone do not tell the matches
   uint32_t pad;
   unsigned long long build_rows;
   unsigned long long distinct;
@@ -86,6 +112,40 @@ __global__ void __launch_bounds__(kBuildBlock) join_count_kernel(bo_join_build_c
 }
 
 // ------------------------------------------------------------ init -------
+// The key bits of a call: n of them (used from kBitsCapLog2 on), or smem_n for
+// the probe's shared memory; multiples of 128, one of them 0.
+struct KeyBits {
+  uint32_t* bits = nullptr;
+  uint32_t n = 0, smem_n = 0;
+};
+
+// Clears the table of 2^cl slots, the Bloom filter, the key bits if they are
+// used, and the join state.
+__device__ __forceinline__ void join_clear(unsigned long long* slots, uint32_t* bloom, const KeyBits& kb,
+                                           JoinMeta* meta, int32_t cl) {
+  const uint64_t cap = 1ull << cl;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
+  for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
+  uint4* b4 = reinterpret_cast<uint4*>(bloom);
+  for (uint64_t i = tid; i < kBloomWords / 4; i += stride) b4[i] = make_uint4(0, 0, 0, 0);
+  const uint32_t n_bits = cl < kBitsCapLog2 ? 0u : kb.n;
+  uint4* k4 = reinterpret_cast<uint4*>(kb.bits);
+  for (uint64_t i = tid; i < (n_bits + kb.smem_n) / 128; i += stride) k4[i] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) {
+    meta->cap_log2 = cl;
+    meta->done = 0;
+    meta->overflow = 0;
+    meta->n_bits = n_bits;
+    meta->hashed = 0;
+    meta->build_rows = 0;
+    meta->distinct = 0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) meta->acc[i] = 0;
+  }
+}
+
 // Capacity: host-chosen (exact count) or, when `pred` is given, derived on the
 // device from the predicted qualifying-row count: the smallest power of two
 // >= kPresizeFactor * pred, clamped to [2^kMinCapLog2, 2^max_log2].  Every block
@@ -103,26 +163,9 @@ __device__ __forceinline__ int32_t presize_log2(const float* pred, int32_t host_
   return presize_log2_of(*pred, max_log2);
 }
 
-__global__ void join_init_kernel(unsigned long long* slots, uint32_t* bloom, JoinMeta* meta, const float* pred,
-                                 int32_t host_log2, int32_t max_log2) {
+__global__ void join_init_kernel(unsigned long long* slots, uint32_t* bloom, KeyBits kb, JoinMeta* meta, const float* pred, int32_t host_log2, int32_t max_log2) {
   pdl_launch_dependents();  // the build kernel may be scheduled now (it waits before touching the table)
-  const int32_t cl = presize_log2(pred, host_log2, max_log2);
-  const uint64_t cap = 1ull << cl;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
-  for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
-  uint4* b4 = reinterpret_cast<uint4*>(bloom);
-  for (uint64_t i = tid; i < kBloomWords / 4; i += stride) b4[i] = make_uint4(0, 0, 0, 0);
-  if (tid == 0) {
-    meta->cap_log2 = cl;
-    meta->done = 0;
-    meta->overflow = 0;
-    meta->build_rows = 0;
-    meta->distinct = 0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) meta->acc[i] = 0;
-  }
+  join_clear(slots, bloom, kb, meta, presize_log2(pred, host_log2, max_log2));
 }
 
 // The learned form's first kernel: every block evaluates the sizing MLP for
@@ -134,31 +177,15 @@ __global__ void join_init_kernel(unsigned long long* slots, uint32_t* bloom, Joi
 __global__ void __launch_bounds__(kPredThreads) join_learned_init_kernel(const float* __restrict__ params,
                                                                          FeatureVec xv, int F, int O,
                                                                          unsigned long long* slots, uint32_t* bloom,
-                                                                         JoinMeta* meta, int32_t max_log2,
+                                                                         KeyBits kb, JoinMeta* meta, int32_t max_log2,
                                                                          float* pred_out) {
   __shared__ float y[kMaxO];
   pdl_launch_dependents();  // the build kernel may be scheduled now (it waits before touching the table)
   mlp_predict_block(params, xv, F, O, y);
   const float c = expm1f(y[0]);
   const float pred = c > 0.0f ? c : 0.0f;
-  const int32_t cl = presize_log2_of(pred, max_log2);
-  const uint64_t cap = 1ull << cl;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
-  for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
-  uint4* b4 = reinterpret_cast<uint4*>(bloom);
-  for (uint64_t i = tid; i < kBloomWords / 4; i += stride) b4[i] = make_uint4(0, 0, 0, 0);
-  if (tid == 0) {
-    meta->cap_log2 = cl;
-    meta->done = 0;
-    meta->overflow = 0;
-    meta->build_rows = 0;
-    meta->distinct = 0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) meta->acc[i] = 0;
-    if (pred_out) *pred_out = pred;
-  }
+  join_clear(slots, bloom, kb, meta, presize_log2_of(pred, max_log2));
+  if (pred_out && blockIdx.x == 0 && threadIdx.x == 0) *pred_out = pred;
 }
 
 // ------------------------------------------------------------ K2 build ---
@@ -177,15 +204,16 @@ constexpr int kBuildRowsPerThread = 16;
 template <bool kSparseKeys>
 __global__ void __launch_bounds__(kBuildBlock) join_build_kernel(bo_join_build_cols b, int32_t date_lt, uint32_t seg,
                                                                  unsigned long long* slots, uint32_t* bloom,
-                                                                 JoinMeta* meta, uint64_t probe_limit) {
+                                                                 uint32_t* bits, uint32_t smem_bits, JoinMeta* meta,
+                                                                 uint64_t probe_limit) {
   // Launched right behind the init kernel (programmatic dependent launch):
   // each thread loads and filters its first rows, then waits for the init
   // kernel to finish before it reads the table's size or touches the table.
   pdl_launch_dependents();
   bool waited = false;
   uint64_t mask = 0;
-  uint32_t qual = 0, newkeys = 0;
-  bool full = false;
+  uint32_t qual = 0, newkeys = 0, n_bits = 0;
+  bool full = false, hashed = false;
   __shared__ uint32_t build_q[kBuildBlock / 32][32 * kBuildRowsPerThread];
   const int lane = threadIdx.x & 31;
   uint32_t* bq = build_q[threadIdx.x >> 5];
@@ -240,6 +268,7 @@ __global__ void __launch_bounds__(kBuildBlock) join_build_kernel(bo_join_build_c
       // Read-only for this kernel (written by the init kernel): the L1-cached
       // path avoids every warp hitting the same L2 sector.
       mask = (1ull << __ldg(&meta->cap_log2)) - 1;
+      n_bits = __ldg(&meta->n_bits);
     }
     qual += __popc(q);
     // Compact the qualifying keys of the whole warp into its queue so the CAS
@@ -251,18 +280,31 @@ __global__ void __launch_bounds__(kBuildBlock) join_build_kernel(bo_join_build_c
     for (int k = 0; k < kBuildRowsPerThread; ++k)
       if ((q >> k) & 1u) bq[pos++] = (uint32_t)keys[k];
     __syncwarp();
-    for (uint32_t i = lane; i < total; i += 32) join_insert(slots, bloom, mask, (int32_t)bq[i], newkeys, full, probe_limit);
+    for (uint32_t i = lane; i < total; i += 32) {
+      const uint32_t key = bq[i], bit = 1u << (key & 31u), before = newkeys;
+      uint32_t repeats = 0;
+      if (key >= n_bits) {
+        join_insert(slots, bloom, mask, (int32_t)key, newkeys, full, probe_limit);
+        if (key < smem_bits) atomicOr(bits + (key >> 5), bit);
+        hashed |= key >= smem_bits || newkeys == before;
+      } else if (!(atomicOr(bits + (key >> 5), bit) & bit)) {
+        ++newkeys;
+      } else {
+        join_insert(slots, bloom, mask, (int32_t)key, repeats, full, probe_limit);  // a key counted already
+        hashed = true;
+      }
+    }
     __syncwarp();
   }
   if (!waited) pdl_wait();  // threads without rows: before the counters below
   // Block-level totals, then one atomic per counter per block.
   __shared__ uint32_t part[3][kBuildBlock / 32];
   const uint32_t wq = warp_sum_u32(qual), wn = warp_sum_u32(newkeys);
-  const unsigned any_full = __any_sync(0xffffffffu, full);
+  const unsigned any_full = __any_sync(0xffffffffu, full), any_hashed = __any_sync(0xffffffffu, hashed && (n_bits | smem_bits));
   if ((threadIdx.x & 31) == 0) {
     part[0][threadIdx.x >> 5] = wq;
     part[1][threadIdx.x >> 5] = wn;
-    part[2][threadIdx.x >> 5] = any_full;
+    part[2][threadIdx.x >> 5] = (any_full ? 1u : 0u) | (any_hashed ? 2u : 0u);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -278,7 +320,8 @@ __global__ void __launch_bounds__(kBuildBlock) join_build_kernel(bo_join_build_c
       // A presized table is "too small" once it is more than 7/8 occupied.
       if (before + tn > (mask + 1) - ((mask + 1) >> 3)) atomicOr(&meta->overflow, 1u);
     }
-    if (tf) atomicOr(&meta->overflow, 1u);
+    if (tf & 1u) atomicOr(&meta->overflow, 1u);
+    if (tf & 2u) atomicOr(&meta->hashed, 1u);
   }
 }
 
@@ -369,44 +412,106 @@ __device__ __forceinline__ void probe_emit(const int32_t* qf, const uint16_t* qo
   }
 }
 
-template <bool kEmit>
-__global__ void __launch_bounds__(kJoinBlock, 2) join_probe_kernel(bo_join_probe_cols p,
-                                                                const unsigned long long* slots,
-                                                                const uint32_t* bloom_g, JoinMeta* meta,
-                                                                bo_join_result* out, int32_t mode, uint64_t probe_limit,
-                                                                uint32_t* err, EmitOut eo) {
-  extern __shared__ __align__(128) uint32_t bloom_s[];
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ unsigned __int128 red[kJoinBlock + 32];
-  __shared__ int32_t q_fk[kProbeWarps][kQueue];
-  __shared__ uint16_t q_off[kProbeWarps][kQueue];
-  pdl_wait();  // launched behind the build kernel: its table and Bloom filter must be complete
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    mbar_arrive_expect_tx(&bar, kBloomBytes);
-    bulk_copy_g2s(bloom_s, bloom_g, kBloomBytes, &bar);
-  }
-  __syncthreads();
-  // On a (never expected) timeout the filter is simply not used: every row then
-  // probes the table directly, which gives the same answer.
-  const bool use_bloom = mbar_wait_bounded(&bar, 0, kWaitLimitNs);
+// Probe of a table with key bits: lane-strided rows, so that the price and
+// discount loads of matching rows coalesce.  kHashed: some keys, or repeats of
+// keys, are in the hash table, behind the Bloom filter.  Bound by the random
+// bit reads, 195 billion a second from L2.  Not inlined: it would take registers
+// from the hashed probe.
+template <bool kHashed>
+static __device__ __noinline__ ProbeAcc probe_bits(const bo_join_probe_cols p, const uint32_t* __restrict__ bits,
+                                                   uint32_t n_bits, const unsigned long long* slots, uint64_t mask,
+                                                   uint64_t limit, const uint32_t* bl, uint32_t wmask) {
   ProbeAcc acc;
-  if (!use_bloom) acc.bad |= kErrSpinTimeout;
-  __shared__ uint32_t all_ones;
-  if (threadIdx.x == 0) all_ones = 0xffffffffu;
-  __syncthreads();
-  const uint32_t* bl = use_bloom ? bloom_s : &all_ones;
-  const uint32_t wmask = use_bloom ? (kBloomWords - 1u) : 0u;
+  constexpr int kRows = kHashed ? 4 : 8;
+  const int64_t n = p.n_rows, stride = (int64_t)gridDim.x * kJoinBlock * kRows;
+  const int64_t first = ((int64_t)blockIdx.x * kJoinBlock + (threadIdx.x & ~31u)) * kRows + (threadIdx.x & 31);
+  for (int64_t r = first; r < n; r += stride) {
+    uint32_t key[kRows], hit = 0;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) key[j] = r + 32 * j < n ? (uint32_t)__ldcs(p.fk + r + 32 * j) : 0u;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      const bool ok = r + 32 * j < n && key[j] < n_bits;
+      hit |= (ok ? (__ldg(bits + (key[j] >> 5)) >> (key[j] & 31u)) & 1u : 0u) << j;
+    }
+    unsigned long long mult[kRows];
+    if constexpr (kHashed) {
+      unsigned long long v[kRows];
+#pragma unroll
+      for (int j = 0; j < kRows; ++j)
+        v[j] = r + 32 * j < n && bloom_test(bl, wmask, key[j]) ? __ldg(slots + (hash32(key[j]) & mask)) : kEmptySlot;
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) {
+        mult[j] = (hit >> j) & 1u;
+        if (v[j] == kEmptySlot) continue;
+        if ((uint32_t)(v[j] >> 32) == key[j])
+          mult[j] += v[j] & 0xffffffffull;
+        else
+          mult[j] += probe_slow<false>(slots, mask, hash32(key[j]) & mask, key[j], limit);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kRows; ++j) mult[j] = (hit >> j) & 1u;
+    }
+    uint64_t pr[kRows], dc[kRows];
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+      pr[j] = mult[j] ? (uint64_t)__ldcs(p.price + r + 32 * j) : 0;
+      dc[j] = mult[j] ? (uint64_t)__ldcs(p.discount + r + 32 * j) : 0;
+    }
+#pragma unroll
+    for (int j = 0; j < kRows; ++j)
+      if (mult[j]) accumulate_match(pr[j], dc[j], mult[j], acc);
+  }
+  return acc;
+}
 
-  const int32_t cl = __ldg(&meta->cap_log2);
-  const uint64_t mask = (1ull << cl) - 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t* qf = q_fk[warp];
-  uint16_t* qo = q_off[warp];
+// The block's totals into the join's, and the result record from the last block.
+__device__ __forceinline__ bool probe_finish(const ProbeAcc& acc, unsigned __int128* red, JoinMeta* meta,
+                                             bo_join_result* out, int32_t mode, uint32_t* err) {
+  if (acc.bad) raise_error(err, acc.bad);
+  const unsigned __int128 bc = block_sum_u128(acc.cnt, red);
+  const unsigned __int128 bt = block_sum_u128(acc.tsum, red);
+  const unsigned __int128 br = block_sum_u128(acc.rsum, red);
+  if (threadIdx.x == 0) {
+    if (bc) atomic_add_i128(&meta->acc[0], (__int128)bc);
+    if (bt) atomic_add_i128(&meta->acc[2], (__int128)bt);
+    if (br) atomic_add_i128(&meta->acc[4], (__int128)br);
+  }
+  if (!last_block(&meta->done)) return false;
+  if (threadIdx.x == 0) {
+    uint32_t fbad = 0;
+    const __int128 m = load_i128(&meta->acc[0]), t = load_i128(&meta->acc[2]), rr = load_i128(&meta->acc[4]);
+    bo_join_result res;
+    res.build_rows = (int64_t)__ldcg(&meta->build_rows);
+    res.distinct_keys = (int64_t)__ldcg(&meta->distinct);
+    res.match_count = narrow_i64(m, fbad);
+    res.sum_trunc = to_bo_i128(t);
+    res.sum_exact = to_bo_i128(t * 100 + rr);
+    res.capacity_log2 = __ldg(&meta->cap_log2);
+    res.overflowed = (int32_t)__ldcg(&meta->overflow);
+    res.reruns = 0;
+    res.mode = mode;
+    *out = res;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) meta->acc[i] = 0;
+    meta->done = 0;
+    if (fbad) raise_error(err, fbad);
+  }
+  return true;
+}
+
+// The rows of this block's warps through the filter and the table; qf and qo
+// are this warp's queue.
+template <bool kEmit>
+__device__ __forceinline__ void probe_hashed(const bo_join_probe_cols& p, const unsigned long long* slots,
+                                             uint64_t mask, uint64_t probe_limit, const uint32_t* bl, uint32_t wmask,
+                                             int32_t* qf, uint16_t* qo, const EmitOut& eo, ProbeAcc& acc) {
+  const int lane = threadIdx.x & 31;
   const int64_t n = p.n_rows;
   const int64_t steps = (n + kRowsPerWarpStep - 1) / kRowsPerWarpStep;
-  const int64_t nwarps = (int64_t)gridDim.x * kProbeWarps;
-  for (int64_t st = (int64_t)blockIdx.x * kProbeWarps + warp; st < steps; st += nwarps) {
+  const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t st = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); st < steps; st += nwarps) {
     const int64_t base = st * kRowsPerWarpStep;
     const int64_t r0 = base + lane * kRowsPerLane;
     int32_t fk[kRowsPerLane];
@@ -448,47 +553,181 @@ __global__ void __launch_bounds__(kJoinBlock, 2) join_probe_kernel(bo_join_probe
       probe_resolve<kJoinResolveR, false>(qf, qo, total, base, slots, mask, probe_limit, p.price, p.discount, acc);
     __syncwarp();
   }
+}
+
+// kBits: the table may have key bits.
+template <bool kEmit, bool kBits>
+__global__ void __launch_bounds__(kJoinBlock, 2) join_probe_kernel(bo_join_probe_cols p,
+                                                                const unsigned long long* slots,
+                                                                const uint32_t* bloom_g,
+                                                                const uint32_t* __restrict__ bits, JoinMeta* meta,
+                                                                bo_join_result* out, int32_t mode, uint64_t probe_limit,
+                                                                uint32_t* err, EmitOut eo) {
+  extern __shared__ __align__(128) uint32_t bloom_s[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ unsigned __int128 red[kProbeWarps];
+  __shared__ int32_t q_fk[kProbeWarps][kQueue];
+  __shared__ uint16_t q_off[kProbeWarps][kQueue];
+  pdl_wait();  // launched behind the build kernel: its table and Bloom filter must be complete
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    mbar_arrive_expect_tx(&bar, kBloomBytes);
+    bulk_copy_g2s(bloom_s, bloom_g, kBloomBytes, &bar);
+  }
+  __syncthreads();
+  // On a (never expected) timeout the filter is simply not used: every row then
+  // probes the table directly, which gives the same answer.
+  const bool use_bloom = mbar_wait_bounded(&bar, 0, kWaitLimitNs);
+  ProbeAcc acc;
+  if (!use_bloom) acc.bad |= kErrSpinTimeout;
+  __shared__ uint32_t all_ones;
+  if (threadIdx.x == 0) all_ones = 0xffffffffu;
+  __syncthreads();
+  const uint32_t* bl = use_bloom ? bloom_s : &all_ones;
+  const uint32_t wmask = use_bloom ? (kBloomWords - 1u) : 0u;
+  const uint64_t mask = (1ull << __ldg(&meta->cap_log2)) - 1;
+  const uint32_t n_bits = kBits ? __ldg(&meta->n_bits) : 0u;
+  if (n_bits) {
+    const uint32_t bad = acc.bad;
+    acc = __ldg(&meta->hashed) ? probe_bits<true>(p, bits, n_bits, slots, mask, probe_limit, bl, wmask)
+                               : probe_bits<false>(p, bits, n_bits, slots, mask, probe_limit, bl, wmask);
+    acc.bad |= bad;
+  } else {
+    probe_hashed<kEmit>(p, slots, mask, probe_limit, bl, wmask, q_fk[threadIdx.x >> 5], q_off[threadIdx.x >> 5], eo,
+                        acc);
+  }
   if (!use_bloom) {
     // The bulk copy may still be in flight: wait for it (bounded) before exit.
     mbar_wait_bounded(&bar, 0, kWaitLimitNs);
   }
-  if (acc.bad) raise_error(err, acc.bad);
-  const unsigned long long cnt = acc.cnt, rsum = acc.rsum;
-  const unsigned __int128 tsum = acc.tsum;
-
-  const unsigned __int128 bc = block_sum_u128(cnt, red);
-  const unsigned __int128 bt = block_sum_u128(tsum, red);
-  const unsigned __int128 br = block_sum_u128(rsum, red);
-  if (threadIdx.x == 0) {
-    if (bc) atomic_add_i128(&meta->acc[0], (__int128)bc);
-    if (bt) atomic_add_i128(&meta->acc[2], (__int128)bt);
-    if (br) atomic_add_i128(&meta->acc[4], (__int128)br);
-  }
-  if (last_block(&meta->done)) {
-    if (threadIdx.x == 0) {
-      uint32_t fbad = 0;
-      const __int128 m = load_i128(&meta->acc[0]), t = load_i128(&meta->acc[2]), rr = load_i128(&meta->acc[4]);
-      bo_join_result res;
-      res.build_rows = (int64_t)__ldcg(&meta->build_rows);
-      res.distinct_keys = (int64_t)__ldcg(&meta->distinct);
-      res.match_count = narrow_i64(m, fbad);
-      res.sum_trunc = to_bo_i128(t);
-      res.sum_exact = to_bo_i128(t * 100 + rr);
-      res.capacity_log2 = cl;
-      res.overflowed = (int32_t)__ldcg(&meta->overflow);
-      res.reruns = 0;
-      res.mode = mode;
-      *out = res;
-#pragma unroll
-      for (int i = 0; i < 6; ++i) meta->acc[i] = 0;
-      meta->done = 0;
-      if constexpr (kEmit) {
-        const uint32_t entries = atomicExch(eo.counter, 0u);
-        *reinterpret_cast<volatile uint32_t*>(eo.count_host) = entries < eo.capacity ? entries : eo.capacity;
-      }
-      if (fbad) raise_error(err, fbad);
+  const bool last = probe_finish(acc, red, meta, out, mode, err);
+  if constexpr (kEmit) {
+    if (last && threadIdx.x == 0) {
+      const uint32_t entries = atomicExch(eo.counter, 0u);
+      *reinterpret_cast<volatile uint32_t*>(eo.count_host) = entries < eo.capacity ? entries : eo.capacity;
     }
   }
+}
+
+// Probe with all key bits in shared memory (kSmemBits), one block per SM.  A
+// warp requests its first two steps' fk before it waits for the build, and
+// each further step two steps ahead; its matches queue up across steps until
+// 64 of them load their price and discount together.  Bound by latency at 6M
+// rows (five steps a warp): the copy of the bits, the payload's round trips and
+// the block totals; 70 MB of DRAM reads, sparse payload among them, are 11 us.
+constexpr int kSmemBlock = 1024;
+constexpr int kSmemWarps = kSmemBlock / 32;
+constexpr uint32_t kSmemFlushAt = 64;
+constexpr int kSmemQueue = (int)kSmemFlushAt + kRowsPerWarpStep;  // matches per warp: (step, row of the step)
+constexpr size_t kSmemQueueBytes = (size_t)kSmemWarps * kSmemQueue * 2;
+
+// Dynamic shared memory: the bits, a zero word for keys beyond them and the
+// queues; or, for a table that needs them, the filter and its queues.
+size_t smem_probe_bytes(uint32_t n_bits) {
+  return std::max((size_t)n_bits / 8 + 16 + kSmemQueueBytes, (size_t)kBloomBytes + (size_t)kSmemWarps * kQueue * 6);
+}
+
+__global__ void __launch_bounds__(kSmemBlock, 1) join_probe_smem_kernel(bo_join_probe_cols p,
+                                                                     const unsigned long long* slots,
+                                                                     const uint32_t* bloom_g,
+                                                                     const uint32_t* __restrict__ bits, uint32_t n_bits,
+                                                                     JoinMeta* meta, bo_join_result* out, int32_t mode,
+                                                                     uint64_t probe_limit, uint32_t* err) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ unsigned __int128 red[kSmemWarps];
+  __shared__ uint32_t all_ones;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t n = p.n_rows;
+  const int64_t steps = (n + kRowsPerWarpStep - 1) / kRowsPerWarpStep;
+  const int64_t nwarps = (int64_t)gridDim.x * kSmemWarps, first = (int64_t)blockIdx.x * kSmemWarps + warp;
+  int64_t st = first;
+  auto load = [&](int64_t at, uint32_t (&fk)[kRowsPerLane]) {  // past the end: no key
+    const int64_t r0 = at * kRowsPerWarpStep + lane * kRowsPerLane;
+    if (r0 + kRowsPerLane <= n) {
+      const int8v f = ld_first_v8(p.fk + r0);
+#pragma unroll
+      for (int k = 0; k < kRowsPerLane; ++k) fk[k] = (uint32_t)f.v[k];
+    } else {
+#pragma unroll
+      for (int k = 0; k < kRowsPerLane; ++k) fk[k] = r0 + k < n ? (uint32_t)p.fk[r0 + k] : 0xffffffffu;
+    }
+  };
+  uint32_t f1[kRowsPerLane], f2[kRowsPerLane];
+  load(st, f1);
+  load(st + nwarps, f2);
+  pdl_wait();  // launched behind the build kernel
+  const bool hashed = __ldg(&meta->hashed) != 0;
+  if (threadIdx.x == 0) {
+    const uint32_t bytes = hashed ? kBloomBytes : n_bits / 8;
+    mbar_init(&bar, 1);
+    mbar_arrive_expect_tx(&bar, bytes);
+    bulk_copy_g2s(smem, hashed ? bloom_g : bits, bytes, &bar);
+    all_ones = 0xffffffffu;
+    if (!hashed) smem[n_bits / 32] = 0;
+  }
+  __syncthreads();
+  const bool copied = mbar_wait_bounded(&bar, 0, kWaitLimitNs);
+  ProbeAcc acc;
+  if (!copied) acc.bad |= kErrSpinTimeout;
+  __syncthreads();
+  if (hashed) {
+    const uint64_t mask = (1ull << __ldg(&meta->cap_log2)) - 1;
+    int32_t* qf = reinterpret_cast<int32_t*>(smem + kBloomWords) + warp * kQueue;
+    uint16_t* qo = reinterpret_cast<uint16_t*>(smem + kBloomWords + kSmemWarps * kQueue) + warp * kQueue;
+    probe_hashed<false>(p, slots, mask, probe_limit, copied ? smem : &all_ones, copied ? kBloomWords - 1u : 0u, qf, qo,
+                        EmitOut(), acc);
+  } else if (copied) {  // (otherwise the call ends with an error)
+    uint16_t* q = reinterpret_cast<uint16_t*>(smem + n_bits / 32 + 4) + warp * kSmemQueue;
+    uint32_t qn = 0, age = 0;  // age: steps since the queue was empty
+    int64_t q0 = st;
+    auto resolve = [&]() {
+      __syncwarp();
+      for (uint32_t i0 = 0; i0 < qn; i0 += 64) {
+        uint64_t pr[2], dc[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t i = i0 + 32 * r + lane, e = i < qn ? q[i] : 0u;
+          const int64_t row = (q0 + (int64_t)(e >> 8) * nwarps) * kRowsPerWarpStep + (e & 255u);
+          pr[r] = i < qn ? (uint64_t)__ldg(p.price + row) : 0;
+          dc[r] = i < qn ? (uint64_t)__ldg(p.discount + row) : 0;
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (i0 + 32 * r + lane < qn) accumulate_match(pr[r], dc[r], 1ull, acc);
+      }
+      qn = 0;
+      __syncwarp();
+    };
+    auto step = [&](uint32_t (&fk)[kRowsPerLane]) {
+      uint32_t hit = 0;
+#pragma unroll
+      for (int k = kRowsPerLane - 1; k >= 0; --k) {
+        const uint32_t x = smem[min(fk[k], n_bits) >> 5];
+        hit = (hit << 1) | (__funnelshift_r(x, x, fk[k]) & 1u);
+      }
+      load(st + 2 * nwarps, fk);
+      uint32_t total;
+      uint32_t pos = qn + warp_exclusive_scan(__popc(hit), total);
+#pragma unroll
+      for (int k = 0; k < kRowsPerLane; ++k)
+        if ((hit >> k) & 1u) q[pos++] = (uint16_t)(age << 8 | (uint32_t)(lane * kRowsPerLane + k));
+      qn += total;
+      st += nwarps;
+      if (qn >= kSmemFlushAt || ++age == 256) {
+        resolve();
+        age = 0;
+        q0 = st;
+      }
+    };
+    while (st < steps) {
+      step(f1);
+      if (st < steps) step(f2);
+    }
+    if (qn) resolve();
+  }
+  if (!copied) mbar_wait_bounded(&bar, 0, kWaitLimitNs);  // the copy may still be in flight
+  probe_finish(acc, red, meta, out, mode, err);
 }
 
 // Host-gather form, second half: the payload of a probe launch's matches,
@@ -537,6 +776,7 @@ namespace {
 struct JoinWs {
   unsigned long long* slots;
   uint32_t* bloom;
+  KeyBits kb;
   JoinMeta* meta;
   float* pred;
   int32_t max_log2;
@@ -563,6 +803,22 @@ int join_workspace(bo_ctx* ctx, int64_t n_build, JoinWs* ws) {
   ws->pred = reinterpret_cast<float*>(static_cast<char*>(p) + sizeof(JoinMeta));
   ws->max_log2 = max_log2;
   return BO_OK;
+}
+
+// Key bits of a call with device columns; where their memory cannot be had,
+// keys are only hashed.
+void join_key_bits(bo_ctx* ctx, int64_t n_build, JoinWs* ws) {
+  auto round128 = [](int64_t v) { return (v + 127) / 128 * 128; };
+  const bool smem = n_build <= kSmemBits;
+  const int64_t n = smem ? std::min(round128(4 * std::max<int64_t>(n_build, 1)), kSmemBits)
+                         : std::min(round128(kBitsPerRow * n_build), int64_t(1) << 31);
+  void* p = nullptr;
+  if (region(ctx, "join_key_bits", (size_t)n / 8, &p) != BO_OK) {
+    cudaGetLastError();
+    return;
+  }
+  ws->kb.bits = static_cast<uint32_t*>(p);
+  (smem ? ws->kb.smem_n : ws->kb.n) = (uint32_t)n;
 }
 
 int check_join(bo_ctx* ctx, const bo_join_build_cols* b, const bo_join_probe_cols* p, const bo_join_params* prm) {
@@ -595,23 +851,41 @@ int grid_for(bo_ctx* ctx, const void* k, int block, size_t smem, int64_t work_it
 int launch_probe(bo_ctx* ctx, const bo_join_probe_cols& p, const JoinWs& ws, bo_join_result* out, int32_t mode,
                  uint64_t probe_limit, bool dependent = false, const EmitOut& eo = EmitOut()) {
   const bool emit = eo.rows != nullptr;
-  auto* kfn = emit ? &join_probe_kernel<true> : &join_probe_kernel<false>;
+  if (ws.kb.smem_n) {
+    const size_t smem = smem_probe_bytes(ws.kb.smem_n);
+    static bool smem_ready = false;
+    if (!smem_ready) {
+      BO_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(&join_probe_smem_kernel),
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_probe_bytes(kSmemBits)));
+      smem_ready = true;
+    }
+    const int64_t steps = (p.n_rows + kRowsPerWarpStep - 1) / kRowsPerWarpStep;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ctx->num_sms, (steps + kSmemWarps - 1) / kSmemWarps));
+    BO_CUDA(ctx, launch_dependent(&join_probe_smem_kernel, grid, kSmemBlock, smem, ctx->stream, p,
+                                  (const unsigned long long*)ws.slots, (const uint32_t*)ws.bloom,
+                                  (const uint32_t*)ws.kb.bits, ws.kb.smem_n, ws.meta, out, mode, probe_limit,
+                                  ctx->d_err));
+    return after_launch(ctx, "join_probe_smem_kernel");
+  }
+  const int form = emit ? 0 : ws.kb.bits ? 1 : 2;
+  auto* kfn = emit ? &join_probe_kernel<true, false>
+                   : ws.kb.bits ? &join_probe_kernel<false, true> : &join_probe_kernel<false, false>;
   const void* k = reinterpret_cast<const void*>(kfn);
-  static bool ready[2] = {false, false};
-  if (!ready[emit]) {
+  static bool ready[3] = {false, false, false};
+  if (!ready[form]) {
     BO_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBloomBytes));
-    ready[emit] = true;
+    ready[form] = true;
   }
   // Enough blocks to fill the GPU, but each thread should see a few 8-row
   // chunks so the per-block Bloom-filter copy is amortised.
   const int grid = grid_for(ctx, k, kJoinBlock, kBloomBytes, (p.n_rows + kRowsPerLane - 1) / kRowsPerLane);
   if (dependent)
     BO_CUDA(ctx, launch_dependent(kfn, grid, kJoinBlock, kBloomBytes, ctx->stream, p,
-                                  (const unsigned long long*)ws.slots, (const uint32_t*)ws.bloom, ws.meta, out, mode,
-                                  probe_limit, ctx->d_err, eo));
+                                  (const unsigned long long*)ws.slots, (const uint32_t*)ws.bloom,
+                                  (const uint32_t*)ws.kb.bits, ws.meta, out, mode, probe_limit, ctx->d_err, eo));
   else
-    kfn<<<grid, kJoinBlock, kBloomBytes, ctx->stream>>>(p, ws.slots, ws.bloom, ws.meta, out, mode, probe_limit,
-                                                        ctx->d_err, eo);
+    kfn<<<grid, kJoinBlock, kBloomBytes, ctx->stream>>>(p, ws.slots, ws.bloom, ws.kb.bits, ws.meta, out, mode,
+                                                        probe_limit, ctx->d_err, eo);
   return after_launch(ctx, "join_probe_kernel");
 }
 
@@ -620,7 +894,8 @@ int join_run(bo_ctx* ctx, const bo_join_build_cols& b, const bo_join_probe_cols&
              const JoinWs& ws, const float* pred, int32_t host_log2, bo_join_result* out, int32_t mode) {
   const void* ki = reinterpret_cast<const void*>(&join_init_kernel);
   const int gi = grid_for(ctx, ki, 256, 0, (int64_t)1 << std::min(ws.max_log2, 24));
-  join_init_kernel<<<gi, 256, 0, ctx->stream>>>(ws.slots, ws.bloom, ws.meta, pred, host_log2, ws.max_log2);
+  join_init_kernel<<<gi, 256, 0, ctx->stream>>>(ws.slots, ws.bloom, ws.kb, ws.meta, pred, host_log2,
+                                                ws.max_log2);
   int rc = after_launch(ctx, "join_init_kernel");
   if (rc) return rc;
   const void* kb = reinterpret_cast<const void*>(&join_build_kernel<false>);
@@ -628,7 +903,8 @@ int join_run(bo_ctx* ctx, const bo_join_build_cols& b, const bo_join_probe_cols&
   // Exact-size tables (mode 0) probe without a bound; presized ones fail fast.
   const uint64_t limit = mode == 0 ? ~0ull : kPresizedProbeLimit;
   BO_CUDA(ctx, launch_dependent(&join_build_kernel<false>, gb, kBuildBlock, 0, ctx->stream, b, prm.date_lt,
-                                (uint32_t)prm.segment_eq, ws.slots, ws.bloom, ws.meta, limit));
+                                (uint32_t)prm.segment_eq, ws.slots, ws.bloom, ws.kb.bits, ws.kb.smem_n, ws.meta,
+                                limit));
   if ((rc = after_launch(ctx, "join_build_kernel"))) return rc;
   return launch_probe(ctx, p, ws, out, mode, limit, true);
 }
@@ -642,6 +918,7 @@ int join_plain_impl(bo_ctx* ctx, const bo_join_build_cols& b, const bo_join_prob
   JoinWs ws;
   int rc = join_workspace(ctx, b.n_rows, &ws);
   if (rc) return rc;
+  join_key_bits(ctx, b.n_rows, &ws);
   // K7: exact count, then one host round trip to size the table.
   BO_CUDA(ctx, cudaMemsetAsync(&ws.meta->count, 0, sizeof(unsigned long long), ctx->stream));
   const void* kc = reinterpret_cast<const void*>(&join_count_kernel);
@@ -802,13 +1079,13 @@ int stream_compute(bo_ctx* ctx, const bo_join_build_cols* bh, const bo_join_prob
   const bo_join_build_cols b = {in.key, s.date, s.seg, nb};
   const void* ki = reinterpret_cast<const void*>(&join_init_kernel);
   join_init_kernel<<<grid_for(ctx, ki, 256, 0, (int64_t)1 << std::min(ws.max_log2, 24)), 256, 0, ctx->stream>>>(
-      ws.slots, ws.bloom, ws.meta, pred, host_log2, ws.max_log2);
+      ws.slots, ws.bloom, KeyBits(), ws.meta, pred, host_log2, ws.max_log2);
   int rc = after_launch(ctx, "join_init_kernel");
   if (rc) return rc;
   const void* kb = reinterpret_cast<const void*>(&join_build_kernel<true>);
   join_build_kernel<true><<<grid_for(ctx, kb, kBuildBlock, 0, (nb + kBuildRowsPerThread - 1) / kBuildRowsPerThread),
                       kBuildBlock, 0, ctx->stream>>>(b, prm->date_lt, (uint32_t)prm->segment_eq, ws.slots, ws.bloom,
-                                                     ws.meta, limit);
+                                                     nullptr, 0u, ws.meta, limit);
   if ((rc = after_launch(ctx, "join_build_kernel"))) return rc;
   for (int64_t c = 0; c < in.chunks; ++c) {
     const int64_t lo = c * kStreamChunkRows, n = std::max<int64_t>(0, std::min(np - lo, kStreamChunkRows));
@@ -988,13 +1265,13 @@ int stream_compute_gather(bo_ctx* ctx, GatherState* g, const bo_join_build_cols*
   const bo_join_build_cols b = {in.key, s.date, s.seg, nb};
   const void* ki = reinterpret_cast<const void*>(&join_init_kernel);
   join_init_kernel<<<grid_for(ctx, ki, 256, 0, (int64_t)1 << std::min(ws.max_log2, 24)), 256, 0, ctx->stream>>>(
-      ws.slots, ws.bloom, ws.meta, pred, host_log2, ws.max_log2);
+      ws.slots, ws.bloom, KeyBits(), ws.meta, pred, host_log2, ws.max_log2);
   int rc = after_launch(ctx, "join_init_kernel");
   if (rc) return rc;
   const void* kb = reinterpret_cast<const void*>(&join_build_kernel<true>);
   join_build_kernel<true><<<grid_for(ctx, kb, kBuildBlock, 0, (nb + kBuildRowsPerThread - 1) / kBuildRowsPerThread),
                       kBuildBlock, 0, ctx->stream>>>(b, prm->date_lt, (uint32_t)prm->segment_eq, ws.slots, ws.bloom,
-                                                     ws.meta, limit);
+                                                     nullptr, 0u, ws.meta, limit);
   if ((rc = after_launch(ctx, "join_build_kernel"))) return rc;
   for (int64_t c = 0; c < in.chunks; ++c) {
     const int64_t lo = c * kStreamChunkRows, n = std::max<int64_t>(0, std::min(np - lo, kStreamChunkRows));
@@ -1138,6 +1415,7 @@ int bo_join_presized_device(bo_ctx* ctx, const bo_join_build_cols* b, const bo_j
   if (!pred_device || !out_device) return set_error(ctx, BO_ERR_INVALID, "join: null prediction or output");
   JoinWs ws;
   if ((rc = join_workspace(ctx, b->n_rows, &ws))) return rc;
+  join_key_bits(ctx, b->n_rows, &ws);
   return join_run(ctx, *b, *p, *prm, ws, pred_device, 0, out_device, 1);
 }
 
@@ -1156,13 +1434,16 @@ int bo_join_learned_device(bo_ctx* ctx, const bo_mlp* m, const float* features_h
   for (int i = 0; i < kMaxF; ++i) fv.f[i] = i < F ? features_host[i] : 0.0f;
   JoinWs ws;
   if ((rc = join_workspace(ctx, b->n_rows, &ws))) return rc;
+  join_key_bits(ctx, b->n_rows, &ws);
   join_learned_init_kernel<<<ctx->num_sms * 2, kPredThreads, 0, ctx->stream>>>(params, fv, F, O, ws.slots, ws.bloom,
-                                                                             ws.meta, ws.max_log2, pred_device);
+                                                                             ws.kb, ws.meta,
+                                                                             ws.max_log2, pred_device);
   if ((rc = after_launch(ctx, "join_learned_init_kernel"))) return rc;
   const void* kb = reinterpret_cast<const void*>(&join_build_kernel<false>);
   const int gb = grid_for(ctx, kb, kBuildBlock, 0, (b->n_rows + kBuildRowsPerThread - 1) / kBuildRowsPerThread);
   BO_CUDA(ctx, launch_dependent(&join_build_kernel<false>, gb, kBuildBlock, 0, ctx->stream, *b, prm->date_lt,
-                                (uint32_t)prm->segment_eq, ws.slots, ws.bloom, ws.meta, (uint64_t)kPresizedProbeLimit));
+                                (uint32_t)prm->segment_eq, ws.slots, ws.bloom, ws.kb.bits, ws.kb.smem_n, ws.meta,
+                                (uint64_t)kPresizedProbeLimit));
   if ((rc = after_launch(ctx, "join_build_kernel"))) return rc;
   return launch_probe(ctx, *p, ws, out_device, 1, kPresizedProbeLimit, true);
 }
@@ -1217,6 +1498,8 @@ int bo_join_probe_device(bo_ctx* ctx, const bo_join_probe_cols* p, bo_join_resul
   JoinWs ws;
   int rc = join_workspace(ctx, 0, &ws);
   if (rc) return rc;
+  auto bits = ctx->regions.find("join_key_bits");
+  if (bits != ctx->regions.end()) ws.kb.bits = static_cast<uint32_t*>(bits->second.ptr);
   return launch_probe(ctx, *p, ws, out_device, 1, ~0ull);  // the table's build bound is not known here
 }
 
