@@ -728,15 +728,17 @@ __global__ void __launch_bounds__(kPartBlock) gb_part_agg_kernel(const uint4* __
 //            there, 32 tag lookups a warp through L1), its hits queue per warp,
 //            and only rows whose code byte confirms them load their a_id.  Many
 //            pass (gd_scan_all_kernel): no filter, every row reads its code byte
-//            and streams its a_id.  The device decides, the other one returns;
+//            and streams its a_id; counts alone take a bit per row from
+//            gd_planes_kernel.  The device decides, the other one returns;
 //   collect  entries of A's ids: groups, joined rows, the k best of each block,
 //            and in the last block the k best of all and the result record;
 //   years    (counts alone) B once more for the smallest years of the k groups.
 // Entries are {count, smallest year} pairs while those stay well inside L2, and
-// counts alone beyond (kGdPairIds): half the memory, half the atomics.
+// counts alone beyond (kGdPairIds) and in the partitioned form, whose calls have
+// many groups: half the memory, half the atomics, no code bytes.
 // Measured (B200, device time): A 2.5M, B 36M, C 4M, 1% of C: 92 us (cfilter 12,
 // scan 54, collect 21) against 137 us of the hash form; A 25M, B 60M, C 4M, half
-// of C: 810 against 3300 us partitioned by hash (scan 1810, scatter 800, ...).
+// of C: 560 against 3300 us partitioned by hash (scan 1810, scatter 800, ...).
 constexpr int kGdBlock = 1024;
 constexpr int kGdWarps = kGdBlock / 32;
 constexpr int kGdLog2Words = 15;  // Bloom filter: 2^15 words = 128 KB
@@ -755,8 +757,8 @@ constexpr int64_t kGdFilterRows = 1 << 20;
 // none, so that entries start as zero bytes.
 constexpr uint32_t kGdYearTop = 255;
 // Counts are added to in passes over ids that each have at most this many bytes
-// of them, half of L2 (25M ids, 100 MB: one pass 705 us, two 633, three 705;
-// 12.5M ids, 50 MB: two passes cost 8% of the query).
+// of them, half of L2 (25M ids, 100 MB: the query in one pass 798 us, in two 575,
+// in three 660; 12.5M ids, 50 MB: one 286, two 328).
 constexpr int64_t kGdPassBytes = 64 << 20;
 constexpr int64_t kGdPairIds = 8 << 20;  // 64 MB of pairs: half of L2
 
@@ -1034,17 +1036,80 @@ __global__ void __launch_bounds__(kGdBlock, 1) gd_scan_kernel(bo_gb_b_cols b, in
   if (pass) mbar_wait_bounded(&bar, 0, kWaitLimitNs);  // the copy may still be in flight
 }
 
+// Counts alone: the exact bit of every row's c_id, looked up in shared memory.  A
+// block holds one of `ranges` parts of C's bitmap and tests all rows of its group
+// of that many blocks, which read them at about the same time, so that DRAM
+// delivers them once; its answers are one plane of a bit per row (a byte per lane
+// and step).  60M rows, 4M C rows in three parts: 92 us for the planes, bound by
+// the three lookups a row in shared memory, and 2 x 118 us for the passes of
+// gd_scan_all_kernel over them; with lookups through L1 those took 633 us, of
+// which the atomics were 65.  20M rows, 1.3M C rows: 356 -> 212 us the query, 10M:
+// 221 -> 165.
+constexpr int kGpBlock = 1024;
+constexpr int64_t kGpRangeBits = 1600 * 1024;  // 200 KB of shared memory
+constexpr int kGpMaxRanges = 4;
+
+__global__ void __launch_bounds__(kGpBlock, 1)
+    gd_planes_kernel(bo_gb_b_cols b, int64_t n_c, const uint32_t* __restrict__ cbits, uint32_t ranges, uint32_t range,
+                     const GbMeta* __restrict__ meta, bool has_filter, uint8_t* __restrict__ planes,
+                     int64_t plane_bytes) {
+  extern __shared__ __align__(128) uint32_t gp_bits[];  // `range` bits, a multiple of 128, and a zero word
+  pdl_launch_dependents();
+  const uint32_t part = blockIdx.x % ranges, lo = part * range;
+  const int64_t steps = (b.n_rows + 255) / 256;
+  const int64_t nwarps = (int64_t)(gridDim.x / ranges) * (kGpBlock / 32);
+  int64_t st = (int64_t)(blockIdx.x / ranges) * (kGpBlock / 32) + (threadIdx.x >> 5);
+  int32_t n1[8], n2[8];
+  if (st < steps) gd_load8(b.c_id, b.n_rows, st, n1);
+  if (st + nwarps < steps) gd_load8(b.c_id, b.n_rows, st + nwarps, n2);
+  pdl_wait();
+  if (gd_filtered(meta, has_filter)) return;
+  const int64_t words = (n_c + 31) / 32 - lo / 32;  // of the bitmap from lo on; none past its end
+  for (int i = threadIdx.x; i < (int)(range / 128); i += kGpBlock) {
+    uint4 v = make_uint4(0, 0, 0, 0);
+    const uint32_t* src = cbits + lo / 32 + 4 * i;
+    if (4 * i + 4 <= words) {
+      v = __ldcg(reinterpret_cast<const uint4*>(src));
+    } else {
+      if (4 * i < words) v.x = __ldcg(src);
+      if (4 * i + 1 < words) v.y = __ldcg(src + 1);
+      if (4 * i + 2 < words) v.z = __ldcg(src + 2);
+    }
+    reinterpret_cast<uint4*>(gp_bits)[i] = v;
+  }
+  if (threadIdx.x == 0) gp_bits[range / 32] = 0;
+  __syncthreads();
+  uint8_t* plane = planes + part * plane_bytes + (threadIdx.x & 31);
+  auto step = [&](int32_t (&cid)[8]) {
+    uint32_t hit = 0;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+      const uint32_t off = min((uint32_t)cid[k] - lo, range);
+      const uint32_t x = gp_bits[off >> 5];
+      hit = (hit << 1) | (__funnelshift_r(x, x, off) & 1u);
+    }
+    plane[st * 32] = (uint8_t)hit;
+    if (st + 2 * nwarps < steps) gd_load8(b.c_id, b.n_rows, st + 2 * nwarps, cid);
+    st += nwarps;
+  };
+  while (st < steps) {
+    step(n1);
+    if (st < steps) step(n2);
+  }
+}
+
 // Every row: its code byte (random, from L2), its a_id (streamed), its atomics.
-// Counts alone need no year, so a bit of the exact bitmap does, an eighth of
-// the bytes, of which L1 keeps a good part.  Bound by one L1-to-L2 request per
-// cycle and SM (50% busy): 633 us for 60M rows of which half join (740 us with
-// code bytes, in one pass over all ids).
+// Counts alone need no year, so a bit of the exact bitmap does, an eighth of the
+// bytes, or (kPlanes) the answers of gd_planes_kernel; then L2 bounds it (63 %
+// busy with a quarter of the rows' atomics a pass; requesting a step ahead in
+// more registers and fewer warps: 563 -> 598 us the query).
 constexpr int kGaBlock = 256;
 
-template <bool kYear>
+template <bool kYear, bool kPlanes>
 __global__ void __launch_bounds__(kGaBlock, 8)
     gd_scan_all_kernel(bo_gb_b_cols b, int64_t n_c, int32_t id_lo, int32_t id_hi, const uint8_t* __restrict__ code,
-                       const uint32_t* __restrict__ cbits, const GbMeta* __restrict__ meta, bool has_filter,
+                       const uint32_t* __restrict__ cbits, const uint8_t* __restrict__ planes, uint32_t ranges,
+                       int64_t plane_bytes, const GbMeta* __restrict__ meta, bool has_filter,
                        uint32_t* __restrict__ entries) {
   pdl_launch_dependents();
   pdl_wait();
@@ -1060,12 +1125,33 @@ __global__ void __launch_bounds__(kGaBlock, 8)
   bool use_local = true;
   for (int64_t st = (int64_t)blockIdx.x * (kGaBlock / 32) + (threadIdx.x >> 5); st < steps; st += nwarps) {
     int32_t cid[8], aid[8];
-    gd_load8(b.c_id, n, st, cid);
+    uint32_t hit = 0;
     gd_load8(b.a_id, n, st, aid);
+    if constexpr (kPlanes) {
+      uint32_t plane[kGpMaxRanges];  // requested together
+#pragma unroll
+      for (uint32_t r = 0; r < (uint32_t)kGpMaxRanges; ++r)
+        plane[r] = r < ranges ? __ldg(planes + r * plane_bytes + st * 32 + (threadIdx.x & 31)) : 0u;
+#pragma unroll
+      for (int r = 0; r < kGpMaxRanges; ++r) hit |= plane[r];
+    } else {
+      gd_load8(b.c_id, n, st, cid);
+    }
+    if (kPlanes && !use_local) {  // few instructions a row: the pass streams
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (((hit >> k) & 1u) && (uint32_t)(aid[k] - id_lo) <= (uint32_t)(id_hi - id_lo)) atomicAdd(entries + aid[k], 1u);
+      continue;
+    }
     uint32_t y[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const bool in = (uint32_t)cid[k] < nc && aid[k] >= id_lo && aid[k] <= id_hi;
+      const bool in_a = aid[k] >= id_lo && aid[k] <= id_hi;
+      if constexpr (kPlanes) {
+        y[k] = in_a ? (hit >> k) & 1u : 0u;
+        continue;
+      }
+      const bool in = in_a && (uint32_t)cid[k] < nc;
       if (kYear) y[k] = in ? __ldg(code + cid[k]) : 0u;
       else y[k] = in ? (__ldg(cbits + (cid[k] >> 5)) >> (cid[k] & 31)) & 1u : 0u;
     }
@@ -1155,7 +1241,7 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
                                                               const uint32_t* __restrict__ amask, GbMeta* meta,
                                                               int32_t year_lo, int k, int wa, unsigned long long cmax,
                                                               uint32_t* __restrict__ part_counts, uint32_t n_parts,
-                                                              uint32_t shift, unsigned long long* __restrict__ cand,
+                                                              unsigned long long* __restrict__ cand,
                                                               bo_gb_result* __restrict__ out) {
   extern __shared__ uint32_t hist[];  // kParts: n_parts counters
   __shared__ unsigned long long buf[kGcBuf];
@@ -1186,10 +1272,12 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
 #pragma unroll
         for (int j = 0; j < 8; ++j) c[j] = (uint32_t)v.v[j];
       }
-      const uint32_t am = __ldg(amask + (id0 >> 5)) >> (id0 & 31);  // id0 is a multiple of eight
+      const uint32_t am = __ldg(amask + (id0 >> 5)) >> (id0 & 31) & 0xffu;  // id0 is a multiple of eight
+      if (am != 0xffu) {
 #pragma unroll
-      for (int j = 0; j < kGcPer; ++j)
-        if (!((am >> j) & 1u)) c[j] = 0;
+        for (int j = 0; j < kGcPer; ++j)
+          if (!((am >> j) & 1u)) c[j] = 0;
+      }
     } else {
 #pragma unroll
       for (int j = 0; j < kGcPer; ++j) {
@@ -1246,18 +1334,24 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
     const uint32_t id0 = (uint32_t)(t * kGcTile) + threadIdx.x * kGcPer;
     // Counts below the limit's cannot be among the best: most threads stop here.
     const unsigned long long need = limit == ~0ull ? 1ull : cmax - (limit >> wa);
-    uint32_t most = 0;
+    uint32_t most = 0, sum = 0;
 #pragma unroll
     for (int j = 0; j < kGcPer; ++j) {
-      groups += c[j] != 0;
-      joined += c[j];
-      most = c[j] > most ? c[j] : most;
-      if (kParts && c[j]) atomicAdd(hist + (shift >= 32 ? 0u : hash32(id0 + j) >> shift), 1u);
+      groups += min(c[j], 1u);
+      sum += c[j];  // at most B's rows
+      most = max(most, c[j]);
+      if (kParts && c[j]) atomicAdd(hist + __umulhi(hash32(id0 + j), n_parts), 1u);  // n_parts: a power of two
     }
+    joined += sum;
     const bool some = most >= need && most > 0;
     unsigned long long key[kGcPer];
+    if (some) {
 #pragma unroll
-    for (int j = 0; j < kGcPer; ++j) key[j] = some && c[j] ? ((cmax - c[j]) << wa) | (id0 + j) : ~0ull;
+      for (int j = 0; j < kGcPer; ++j) key[j] = c[j] ? ((cmax - c[j]) << wa) | (id0 + j) : ~0ull;
+    } else {
+#pragma unroll
+      for (int j = 0; j < kGcPer; ++j) key[j] = ~0ull;
+    }
     if (t + 2 < t1) load(t + 2, c);
     keep(key, t == t0, some);
   };
@@ -1619,7 +1713,7 @@ int gb_dense(bo_ctx* ctx, const bo_gb_a_cols& a, const bo_gb_b_cols& b, const bo
   CatSet cs{};
   cs.n = prm.n_categories;
   for (int i = 0; i < prm.n_categories; ++i) cs.v[i] = prm.categories[i];
-  const bool filter = b.n_rows >= kGdFilterRows, pairs = ids <= kGdPairIds;
+  const bool filter = b.n_rows >= kGdFilterRows, pairs = ids <= kGdPairIds && !parts;
   uint32_t* entries = reinterpret_cast<uint32_t*>(ws.slots);
   const int64_t vecs = (ids * (pairs ? 8 : 4) + 15) / 16;
   const void* kc = reinterpret_cast<const void*>(&gd_cfilter_kernel);
@@ -1643,13 +1737,36 @@ int gb_dense(bo_ctx* ctx, const bo_gb_a_cols& a, const bo_gb_b_cols& b, const bo
     if ((rc = after_launch(ctx, "gd_scan_kernel"))) return rc;
   }
   if (b.n_rows > 0) {
-    const auto ka = pairs ? &gd_scan_all_kernel<true> : &gd_scan_all_kernel<false>;
+    const uint32_t ranges = (uint32_t)((c.n_rows + kGpRangeBits - 1) / kGpRangeBits);
+    const int64_t plane_bytes = steps * 32;
+    void* planes = nullptr;
+    if (!pairs && filter && ranges >= 1 && ranges <= (uint32_t)kGpMaxRanges &&
+        region(ctx, "gb_planes", (size_t)plane_bytes * ranges, &planes) != BO_OK) {
+      cudaGetLastError();
+      planes = nullptr;
+    }
+    if (planes) {
+      const uint32_t range = (uint32_t)(((c.n_rows + ranges - 1) / ranges + 127) / 128 * 128);
+      const size_t smem = range / 8 + 16;
+      static bool planes_ready = false;
+      if (!planes_ready)
+        BO_CUDA(ctx, cudaFuncSetAttribute(reinterpret_cast<const void*>(&gd_planes_kernel),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kGpRangeBits / 8 + 16)));
+      planes_ready = true;
+      BO_CUDA(ctx, launch_dependent(&gd_planes_kernel, ctx->num_sms / (int)ranges * (int)ranges, kGpBlock, smem,
+                                    ctx->stream, b, c.n_rows, (const uint32_t*)ws.cbits, ranges, range,
+                                    (const GbMeta*)meta, filter, static_cast<uint8_t*>(planes), plane_bytes));
+      if ((rc = after_launch(ctx, "gd_planes_kernel"))) return rc;
+    }
+    const auto ka = pairs ? &gd_scan_all_kernel<true, false>
+                          : planes ? &gd_scan_all_kernel<false, true> : &gd_scan_all_kernel<false, false>;
     const int ga = grid_res(ctx, reinterpret_cast<const void*>(ka), kGaBlock, 0, lanes);
     const int64_t passes = pairs ? 1 : (4 * ids + kGdPassBytes - 1) / kGdPassBytes, span = (ids + passes - 1) / passes;
     for (int64_t lo = 0; lo < ids; lo += span) {
       BO_CUDA(ctx, launch_dependent(ka, ga, kGaBlock, 0, ctx->stream, b, c.n_rows, (int32_t)lo,
                                     (int32_t)(std::min(lo + span, ids) - 1), (const uint8_t*)code,
-                                    (const uint32_t*)ws.cbits, (const GbMeta*)meta, filter, entries));
+                                    (const uint32_t*)ws.cbits, (const uint8_t*)planes, ranges, plane_bytes,
+                                    (const GbMeta*)meta, filter, entries));
       if ((rc = after_launch(ctx, "gd_scan_all_kernel"))) return rc;
     }
   }
@@ -1664,7 +1781,7 @@ int gb_dense(bo_ctx* ctx, const bo_gb_a_cols& a, const bo_gb_b_cols& b, const bo
                                       (int)(4u << BO_GB_MAX_LOG2_PARTITIONS)));
   if (parts) kk_ready[pairs] = true;
   BO_CUDA(ctx, launch_dependent(kk, gk, kGcBlock, 4 * (size_t)n_parts, ctx->stream, (const uint32_t*)entries, ids,
-                                amask, meta, prm.year_lo, (int)prm.k, wa, cmax, part_counts, n_parts, shift, cand, out));
+                                amask, meta, prm.year_lo, (int)prm.k, wa, cmax, part_counts, n_parts, cand, out));
   if ((rc = after_launch(ctx, "gd_collect_kernel"))) return rc;
   if (pairs || b.n_rows == 0 || prm.k == 0) return BO_OK;
   const void* ky = reinterpret_cast<const void*>(&gd_years_kernel);
