@@ -15,16 +15,19 @@
 // and query k's rows are those of the classes <= k of its segment.  At most 32
 // classes exist, so a key carries one byte and a matching probe row adds to one
 // class; the queries' totals are sums over classes at the end.
-//   count   one pass: rows per class, and the smallest and largest key; the last
-//           block turns them into each query's qualifying-row count and the union
-//           count (rows of any class), and decides how keys are stored:
+//   range   the smallest and largest key of all build rows decide how keys are
+//           stored:
 //   dense   one byte per key value between the smallest and the largest key,
 //           where that fits the table's memory (sixteen bytes per build row):
 //           15M dense keys are 15 MB that stay in L2;
-//   hash    else slots of key << 32 | class, sized by the union count, behind a
-//           Bloom filter;
+//   count   else one pass: rows per class and the range of their keys alone, for
+//           which the dense form gets a second chance; or
+//   hash    slots of key << 32 | class, sized by the union count (rows of any
+//           class), behind a Bloom filter;
 //   init    clears whichever it is;
-//   build   one pass: rows with a class store it; a key that is already present
+//   build   one pass: rows with a class store it (and, dense, are counted, unless
+//           they have been: each query's qualifying rows follow from the counts,
+//           and the size of the table there would have been); a key already present
 //           (two build rows with one key) cannot carry per-query multiplicities
 //           in one byte, so it marks the whole call for an exact solo rerun of
 //           every query;
@@ -32,10 +35,11 @@
 //           the warp's shared-memory accumulators; blocks add the classes' totals
 //           into 128-bit totals and the last block writes every query's result.
 // The kernels of the form that was not chosen return at once.  Measured (B200,
-// build 15M, probe 60M, 16 queries, dense keys): 478 us a call (count 62, build
-// 108, probe 305) against 2934 us with a query mask per hashed slot and a warp
+// build 15M, probe 60M, 16 queries, dense keys): 433 us a call (range 14, build
+// 113, probe 306; with a counting pass over all columns, 62 us, instead of the
+// range: 478) against 2934 us with a query mask per hashed slot and a warp
 // reduction per query; keys over the whole 32-bit range (hash): 2703 against
-// 2950 us, 25K x 100K rows: 41 and 66 against 77 us.  The line between the forms
+// 2950 us, 25K x 100K rows: 41 and 64 against 77 us.  The line between the forms
 // is the table's memory and no lower: just inside it (keys ten apart) dense
 // takes 885 us for 2 queries, hash 1656 us just outside (twenty apart).
 #include <algorithm>
@@ -76,9 +80,9 @@ struct MqState {
   unsigned long long distinct;
   uint32_t key_max, key_nmin;                // largest key and largest ~key, in unsigned order
   uint32_t base, range;                      // dense: smallest key, key values from it to the largest
-  uint32_t ticket_count, ticket_probe, dup, overflow;
+  uint32_t ticket_range, ticket_count, ticket_probe, dup, overflow;
   int32_t cap_log2, dense;
-  float union_rows;
+  int32_t counted, any;                      // by the counting pass; any row with a class
 };
 
 __device__ __forceinline__ void mq_load_queries(MultiQ& q, const MultiQ& qv) {
@@ -133,47 +137,82 @@ __device__ __forceinline__ void mq_build_rows(const bo_join_build_cols& b, const
   }
 }
 
-// --------------------------------------------------------------- count ---
+// --------------------------------------------------------------- range ---
 constexpr uint32_t kSign = 0x80000000u;  // int32 order as uint32 order
 
-__global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_cols b, MultiQ qv, MqState* st,
-                                                                 uint32_t dense_max) {
-  constexpr int kCopies = 8;  // of each class's counter: lanes of one class spread over them
-  __shared__ MultiQ q;
-  __shared__ uint32_t h[(kMq + 1) * kCopies];
-  __shared__ unsigned long long tot[kMq + 1];
-  mq_load_queries(q, qv);
-  for (int i = threadIdx.x; i < (kMq + 1) * kCopies; i += kMqBuildBlock) h[i] = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
-  uint32_t kmax = 0, nmin = 0;
-  for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
-       c += (int64_t)gridDim.x * kMqBuildBlock) {
-    uint32_t code[kMqBuildRows], key[kMqBuildRows];
-    mq_build_rows(b, q, c * kMqBuildRows, code, key);
-#pragma unroll
-    for (int j = 0; j < kMqBuildRows; ++j) {
-      if (!code[j]) continue;
-      atomicAdd(h + code[j] * kCopies + (lane & (kCopies - 1)), 1u);
-      const uint32_t k = key[j] ^ kSign;
-      kmax = max(kmax, k);
-      nmin = max(nmin, ~k);
-    }
-  }
+// The block's smallest and largest key into the state's.
+__device__ __forceinline__ void mq_take_range(MqState* st, uint32_t kmax, uint32_t nmin) {
   kmax = __reduce_max_sync(0xffffffffu, kmax);
   nmin = __reduce_max_sync(0xffffffffu, nmin);
-  if (lane == 0 && (kmax | nmin)) {
+  if ((threadIdx.x & 31) == 0 && (kmax | nmin)) {
     atomicMax(&st->key_max, kmax);
     atomicMax(&st->key_nmin, nmin);
   }
+}
+
+__device__ __forceinline__ void mq_decide(MqState* st, bool rows, uint32_t dense_max) {
+  const uint32_t lo = ~__ldcg(&st->key_nmin), hi = __ldcg(&st->key_max);
+  const uint64_t range = rows ? (uint64_t)hi - lo + 1 : 0;
+  st->dense = range <= dense_max;
+  st->base = lo ^ kSign;
+  st->range = (uint32_t)range;
+}
+
+__global__ void __launch_bounds__(kMqBuildBlock) mq_range_kernel(bo_join_build_cols b, MqState* st,
+                                                                 uint32_t dense_max) {
+  pdl_launch_dependents();
+  const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
+  uint32_t kmax = 0, nmin = 0;
+  auto take = [&](int32_t key) {
+    const uint32_t k = (uint32_t)key ^ kSign;
+    kmax = max(kmax, k);
+    nmin = max(nmin, ~k);
+  };
+  for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
+       c += (int64_t)gridDim.x * kMqBuildBlock) {
+    const int64_t r0 = c * kMqBuildRows;
+    if (r0 + kMqBuildRows <= b.n_rows) {
+      const int8v k = ld_stream_v8(b.key + r0);
+#pragma unroll
+      for (int j = 0; j < kMqBuildRows; ++j) take(k.v[j]);
+    } else {
+      for (int64_t r = r0; r < b.n_rows; ++r) take(b.key[r]);
+    }
+  }
+  // One pair of atomics per block: thousands of warps on two words serialise in L2.
+  __shared__ uint32_t bmax, bnmin;
+  if (threadIdx.x == 0) bmax = bnmin = 0;
+  __syncthreads();
+  kmax = __reduce_max_sync(0xffffffffu, kmax);
+  nmin = __reduce_max_sync(0xffffffffu, nmin);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&bmax, kmax);
+    atomicMax(&bnmin, nmin);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && (bmax | bnmin)) {
+    atomicMax(&st->key_max, bmax);
+    atomicMax(&st->key_nmin, bnmin);
+  }
+  if (!last_block(&st->ticket_range) || threadIdx.x != 0) return;
+  mq_decide(st, b.n_rows > 0, dense_max);
+  if (!st->dense) st->key_max = st->key_nmin = 0;  // the counting pass tries the keys of rows with a class
+}
+
+// --------------------------------------------------------------- count ---
+constexpr int kMqClassCopies = 8;  // of each class's counter: lanes of one class spread over them
+
+// The block's class counters into the call's, and in the last block each
+// query's qualifying rows, the union's, and the hash table's size.  True there.
+__device__ __forceinline__ bool mq_count_finish(const uint32_t* h, const MultiQ& q, MqState* st, int32_t max_log2) {
+  __shared__ unsigned long long tot[kMq + 1];
   __syncthreads();
   if (threadIdx.x <= kMq) {
     uint32_t t = 0;
-    for (int i = 0; i < kCopies; ++i) t += h[threadIdx.x * kCopies + i];
+    for (int i = 0; i < kMqClassCopies; ++i) t += h[threadIdx.x * kMqClassCopies + i];
     if (t) atomicAdd(st->hist + threadIdx.x, (unsigned long long)t);
   }
-  if (!last_block(&st->ticket_count)) return;
+  if (!last_block(&st->ticket_count)) return false;
   if (threadIdx.x <= kMq) tot[threadIdx.x] = __ldcg(st->hist + threadIdx.x);
   __syncthreads();
   if (threadIdx.x < q.n) {
@@ -186,28 +225,64 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_c
   if (threadIdx.x == 0) {
     unsigned long long u = 0;
     for (int k = 1; k <= kMq; ++k) u += tot[k];
-    const uint32_t lo = ~__ldcg(&st->key_nmin), hi = __ldcg(&st->key_max);
-    const uint64_t range = u ? (uint64_t)hi - lo + 1 : 0;
-    st->union_rows = (float)u;
-    st->dense = range <= dense_max;
-    st->base = lo ^ kSign;
-    st->range = (uint32_t)range;
+    const double want = (double)(float)u * 2.0;  // exact count: load <= 0.5
+    int32_t cl = kMqMinCapLog2;
+    while (cl < max_log2 && (double)(1ull << cl) < want) ++cl;
+    st->cap_log2 = cl;
+    st->any = u != 0;
+  }
+  return true;
+}
+
+// Where the keys of all rows do not fit the dense form: rows per class before
+// the build, and whether the keys of those rows alone fit it.
+__global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_cols b, MultiQ qv, MqState* st,
+                                                                 uint32_t dense_max, int32_t max_log2) {
+  __shared__ MultiQ q;
+  __shared__ uint32_t h[(kMq + 1) * kMqClassCopies];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (__ldcg(&st->dense)) return;
+  mq_load_queries(q, qv);
+  for (int i = threadIdx.x; i < (kMq + 1) * kMqClassCopies; i += kMqBuildBlock) h[i] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
+  uint32_t kmax = 0, nmin = 0;
+  for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
+       c += (int64_t)gridDim.x * kMqBuildBlock) {
+    uint32_t code[kMqBuildRows], key[kMqBuildRows];
+    mq_build_rows(b, q, c * kMqBuildRows, code, key);
+#pragma unroll
+    for (int j = 0; j < kMqBuildRows; ++j) {
+      if (!code[j]) continue;
+      atomicAdd(h + code[j] * kMqClassCopies + (lane & (kMqClassCopies - 1)), 1u);
+      const uint32_t k = key[j] ^ kSign;
+      kmax = max(kmax, k);
+      nmin = max(nmin, ~k);
+    }
+  }
+  mq_take_range(st, kmax, nmin);
+  if (!mq_count_finish(h, q, st, max_log2)) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    st->counted = 1;
+    mq_decide(st, st->any != 0, dense_max);
   }
 }
 
 // ---------------------------------------------------------------- init ---
-__global__ void mq_init_kernel(unsigned long long* slots, uint32_t* bloom, MqState* st, int32_t max_log2) {
-  const double want = (double)st->union_rows * 2.0;  // exact count: load <= 0.5
-  int32_t cl = kMqMinCapLog2;
-  while (cl < max_log2 && (double)(1ull << cl) < want) ++cl;
+__global__ void mq_init_kernel(unsigned long long* slots, uint32_t* bloom, MqState* st) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid == 0) st->cap_log2 = cl;
-  if (st->dense) {
+  if (__ldg(&st->dense)) {
     uint4* v = reinterpret_cast<uint4*>(slots);
-    for (uint64_t i = tid; i < ((uint64_t)st->range + 15) / 16; i += stride) v[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = tid; i < ((uint64_t)__ldg(&st->range) + 15) / 16; i += stride) v[i] = make_uint4(0, 0, 0, 0);
     return;
   }
+  const int32_t cl = __ldg(&st->cap_log2);
   const uint64_t cap = 1ull << cl;
   ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
   for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
@@ -219,11 +294,17 @@ __global__ void mq_init_kernel(unsigned long long* slots, uint32_t* bloom, MqSta
 // Dense: the class byte is ORed into its word, the old byte tells a repeated
 // key; a thread's atomics are all issued before any old value is used.
 __global__ void __launch_bounds__(kMqBuildBlock) mq_build_dense_kernel(bo_join_build_cols b, MultiQ qv,
-                                                                       uint32_t* __restrict__ bytes, MqState* st) {
-  if (!__ldg(&st->dense)) return;
+                                                                       uint32_t* __restrict__ bytes, MqState* st,
+                                                                       int32_t max_log2) {
   __shared__ MultiQ q;
+  __shared__ uint32_t h[(kMq + 1) * kMqClassCopies];
+  pdl_launch_dependents();
   mq_load_queries(q, qv);
+  for (int i = threadIdx.x; i < (kMq + 1) * kMqClassCopies; i += kMqBuildBlock) h[i] = 0;
+  pdl_wait();
+  if (!__ldg(&st->dense)) return;
   __syncthreads();
+  const uint32_t copy = threadIdx.x & (kMqClassCopies - 1);
   const uint32_t base = __ldg(&st->base);
   const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
   uint32_t dup = 0;
@@ -237,9 +318,13 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_build_dense_kernel(bo_join_b
       old[j] = code[j] ? atomicOr(bytes + (off >> 2), code[j] << (8 * (off & 3u))) : 0u;
     }
 #pragma unroll
+    for (int j = 0; j < kMqBuildRows; ++j)
+      if (code[j]) atomicAdd(h + code[j] * kMqClassCopies + copy, 1u);
+#pragma unroll
     for (int j = 0; j < kMqBuildRows; ++j) dup |= (old[j] >> (8 * ((key[j] - base) & 3u))) & 0xffu;
   }
   if (__any_sync(0xffffffffu, dup != 0) && (threadIdx.x & 31) == 0) atomicOr(&st->dup, 1u);
+  if (!__ldg(&st->counted)) mq_count_finish(h, q, st, max_log2);
 }
 
 __device__ __forceinline__ void mq_insert(unsigned long long* slots, uint32_t* bloom, uint64_t mask, int32_t key,
@@ -267,6 +352,8 @@ __device__ __forceinline__ void mq_insert(unsigned long long* slots, uint32_t* b
 __global__ void __launch_bounds__(kMqBuildBlock) mq_build_kernel(bo_join_build_cols b, MultiQ qv,
                                                                  unsigned long long* slots, uint32_t* bloom,
                                                                  MqState* st) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (__ldg(&st->dense)) return;
   __shared__ MultiQ q;
   __shared__ uint32_t queue[kMqBuildBlock / 32][2][32 * kMqBuildRows];
@@ -412,6 +499,8 @@ constexpr int kMqDenseBlock = 256;
 __global__ void __launch_bounds__(kMqDenseBlock) mq_probe_dense_kernel(bo_join_probe_cols p,
                                                                        const uint8_t* __restrict__ bytes, MqState* st,
                                                                        bo_join_result* out, MultiQ qv, uint32_t* err) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (!__ldg(&st->dense)) return;
   constexpr int kWarps = kMqDenseBlock / 32;
   __shared__ __align__(16) MqWarpAcc wa[kWarps];
@@ -497,6 +586,8 @@ __device__ __forceinline__ void mq_resolve(const int32_t* qf, const uint8_t* qo,
 __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_cols p, const unsigned long long* slots,
                                                               const uint32_t* bloom_g, MqState* st,
                                                               bo_join_result* out, MultiQ qv, uint32_t* err) {
+  pdl_launch_dependents();
+  pdl_wait();
   if (__ldg(&st->dense)) return;
   extern __shared__ __align__(128) uint32_t bloom_s[];
   __shared__ __align__(8) uint64_t bar;
@@ -643,24 +734,30 @@ extern "C" int bo_join_multi_device(bo_ctx* ctx, const bo_join_build_cols* b, co
   // Dense form while the key values from smallest to largest fit the table's memory.
   const uint32_t dense_max = (uint32_t)std::min<uint64_t>(sizeof(unsigned long long) << max_log2, 0xfffffff0ull);
   const int64_t chunks = (b->n_rows + kMqBuildRows - 1) / kMqBuildRows;
+  const void* kr = reinterpret_cast<const void*>(&mq_range_kernel);
+  mq_range_kernel<<<mq_grid(ctx, kr, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(*b, st, dense_max);
+  if ((rc = after_launch(ctx, "mq_range_kernel"))) return rc;
   const void* kc = reinterpret_cast<const void*>(&mq_count_kernel);
-  mq_count_kernel<<<mq_grid(ctx, kc, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(*b, q, st, dense_max);
+  BO_CUDA(ctx, launch_dependent(&mq_count_kernel, mq_grid(ctx, kc, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0,
+                                ctx->stream, *b, q, st, dense_max, max_log2));
   if ((rc = after_launch(ctx, "mq_count_kernel"))) return rc;
   const void* ki = reinterpret_cast<const void*>(&mq_init_kernel);
-  mq_init_kernel<<<mq_grid(ctx, ki, 256, 0, (int64_t)1 << std::min(max_log2, 24)), 256, 0, ctx->stream>>>(
-      slots, bloom, st, max_log2);
+  BO_CUDA(ctx, launch_dependent(&mq_init_kernel, mq_grid(ctx, ki, 256, 0, (int64_t)1 << std::min(max_log2, 24)), 256, 0,
+                                ctx->stream, slots, bloom, st));
   if ((rc = after_launch(ctx, "mq_init_kernel"))) return rc;
   const void* kd = reinterpret_cast<const void*>(&mq_build_dense_kernel);
-  mq_build_dense_kernel<<<mq_grid(ctx, kd, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(
-      *b, q, reinterpret_cast<uint32_t*>(slots), st);
+  BO_CUDA(ctx, launch_dependent(&mq_build_dense_kernel, mq_grid(ctx, kd, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0,
+                                ctx->stream, *b, q, reinterpret_cast<uint32_t*>(slots), st, max_log2));
   if ((rc = after_launch(ctx, "mq_build_dense_kernel"))) return rc;
   const void* kb = reinterpret_cast<const void*>(&mq_build_kernel);
-  mq_build_kernel<<<mq_grid(ctx, kb, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0, ctx->stream>>>(*b, q, slots, bloom, st);
+  BO_CUDA(ctx, launch_dependent(&mq_build_kernel, mq_grid(ctx, kb, kMqBuildBlock, 0, chunks), kMqBuildBlock, 0,
+                                ctx->stream, *b, q, slots, bloom, st));
   if ((rc = after_launch(ctx, "mq_build_kernel"))) return rc;
   const int64_t lanes = (p->n_rows + kMqRowsPerLane - 1) / kMqRowsPerLane;
   const void* kq = reinterpret_cast<const void*>(&mq_probe_dense_kernel);
-  mq_probe_dense_kernel<<<mq_grid(ctx, kq, kMqDenseBlock, 0, lanes), kMqDenseBlock, 0, ctx->stream>>>(
-      *p, reinterpret_cast<const uint8_t*>(slots), st, out_device, q, ctx->d_err);
+  BO_CUDA(ctx, launch_dependent(&mq_probe_dense_kernel, mq_grid(ctx, kq, kMqDenseBlock, 0, lanes), kMqDenseBlock, 0,
+                                ctx->stream, *p, reinterpret_cast<const uint8_t*>(slots), st, out_device, q,
+                                ctx->d_err));
   if ((rc = after_launch(ctx, "mq_probe_dense_kernel"))) return rc;
   const void* kp = reinterpret_cast<const void*>(&mq_probe_kernel);
   constexpr size_t smem = kBloomBytes + kMqWarps * sizeof(MqWarpAcc);
@@ -669,8 +766,9 @@ extern "C" int bo_join_multi_device(bo_ctx* ctx, const bo_join_build_cols* b, co
     BO_CUDA(ctx, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ready = true;
   }
-  mq_probe_kernel<<<mq_grid(ctx, kp, kMqBlock, smem, lanes), kMqBlock, smem, ctx->stream>>>(*p, slots, bloom, st,
-                                                                                           out_device, q, ctx->d_err);
+  BO_CUDA(ctx, launch_dependent(&mq_probe_kernel, mq_grid(ctx, kp, kMqBlock, smem, lanes), kMqBlock, smem, ctx->stream,
+                                *p, (const unsigned long long*)slots, (const uint32_t*)bloom, st, out_device, q,
+                                ctx->d_err));
   return after_launch(ctx, "mq_probe_kernel");
 }
 
