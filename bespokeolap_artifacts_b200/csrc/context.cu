@@ -78,13 +78,29 @@ int consume_device_errors(bo_ctx* ctx, uint32_t* bits_out) {
   return BO_OK;
 }
 
+namespace {
+// A result record and the error word to pinned host memory.
+__global__ void __launch_bounds__(256) result_kernel(const uint32_t* __restrict__ record, uint32_t words,
+                                                     const uint32_t* __restrict__ err, uint32_t* host,
+                                                     uint32_t* host_err) {
+  pdl_wait();
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) host[i] = record[i];
+  if (threadIdx.x == 0) *host_err = *err;
+}
+}  // namespace
+
 int read_result(bo_ctx* ctx, const char* op, void* host, const void* dev, size_t bytes) {
   void* stage = nullptr;
   int rc = host_stage(ctx, bytes, &stage);
   if (rc) return rc;
-  BO_CUDA(ctx, cudaMemcpyAsync(stage, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-  uint32_t bits = 0;
-  if ((rc = consume_device_errors(ctx, &bits))) return rc;  // synchronises the stream
+  if ((rc = drain_host_work(ctx))) return rc;
+  BO_CUDA(ctx, launch_dependent(&result_kernel, 1, 256, 0, ctx->stream, static_cast<const uint32_t*>(dev),
+                                (uint32_t)(bytes / 4), (const uint32_t*)ctx->d_err, static_cast<uint32_t*>(stage),
+                                ctx->h_err));
+  if ((rc = after_launch(ctx, "result_kernel"))) return rc;
+  BO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  const uint32_t bits = *ctx->h_err;
+  if (bits) BO_CUDA(ctx, cudaMemsetAsync(ctx->d_err, 0, sizeof(uint32_t), ctx->stream));
   std::memcpy(host, stage, bytes);
   return device_error_status(ctx, bits, op);
 }

@@ -83,9 +83,10 @@ void destroy_host_work(bo_ctx* ctx);
 int after_launch(bo_ctx* ctx, const char* what);
 // Reads and clears the device error word (call only after a stream sync).
 int consume_device_errors(bo_ctx* ctx, uint32_t* bits_out);
-// A call's result record and the error word in one synchronisation: both are
-// copied to pinned memory, so neither copy waits for the other (a copy to
-// pageable memory synchronises by itself: 15 us more per call).
+// A call's result record (whole words) and the error word in one
+// synchronisation: a kernel right behind the call's last one writes both to
+// pinned memory (two copies there took 8 us more per call, and one to pageable
+// memory, which synchronises by itself, another 15).
 int read_result(bo_ctx* ctx, const char* op, void* host, const void* dev, size_t bytes);
 // Maps error bits to a status code with a message.
 int device_error_status(bo_ctx* ctx, uint32_t bits, const char* op);
