@@ -33,11 +33,15 @@
 
 namespace bo {
 
-// Storage-plan layout: words per group
-//   0 price  1 dp  2 dp*(100+t)  3 p*(100-d)  4 p*(100-d)*(100+t)
-//   5 packed = count | disc << 9 | (qty + 32768) << 25
-// (<= 256 rows: count < 2^9, disc sum < 2^16, offset qty sum < 2^24).
-constexpr int kNarrowWords = 6;
+// Storage-plan layout: words per group, each of a signed field over an unsigned
+// one of kNarrowLow bits (256 rows a thread fill at most those, and the signed
+// ones what is left):
+//   0 price | qty + 32768   1 dp | disc   2 p*d | count   3 dp*t   4 p*(100-d)*t
+// Shared memory bounds the scan: each word moves 16 bytes a row there (6.0M rows
+// with six words, one of them three fields: 28.7 us, with five 26.4).
+constexpr int kNarrowWords = 5;
+constexpr int kNarrowPacked = 3;  // the first words, with a lower field
+__device__ __forceinline__ constexpr int narrow_low(int w) { return w == 0 ? 24 : w == 1 ? 16 : 9; }
 
 __device__ __forceinline__ void narrow_row(unsigned long long* col, int32_t ship, int32_t cutoff, uint32_t code,
                                            int32_t p, int32_t dprice, uint32_t d, uint32_t t, int32_t q,
@@ -47,16 +51,12 @@ __device__ __forceinline__ void narrow_row(unsigned long long* col, int32_t ship
     bad |= kErrBadGroupCode;
     return;
   }
-  const int32_t tm = 100 + (int32_t)t;
-  const int64_t v1 = (int64_t)p * (100 - (int32_t)d);
   unsigned long long* w = col + code * (kNarrowWords * kScanBlock);
-  red_shared_u64(w, (unsigned long long)(int64_t)p);
-  red_shared_u64(w + kScanBlock, (unsigned long long)(int64_t)dprice);
-  red_shared_u64(w + 2 * kScanBlock, (unsigned long long)((int64_t)dprice * tm));
-  red_shared_u64(w + 3 * kScanBlock, (unsigned long long)v1);
-  red_shared_u64(w + 4 * kScanBlock, (unsigned long long)(v1 * tm));
-  red_shared_u64(w + 5 * kScanBlock, 1ull | ((unsigned long long)d << 9) |
-                                         ((unsigned long long)(uint32_t)(q + 32768) << 25));
+  red_shared_u64(w, (unsigned long long)((int64_t)p * (1 << 24) + (q + 32768)));
+  red_shared_u64(w + kScanBlock, (unsigned long long)((int64_t)dprice * (1 << 16) + d));
+  red_shared_u64(w + 2 * kScanBlock, (unsigned long long)((int64_t)p * (int32_t)(d << 9) + 1));
+  red_shared_u64(w + 3 * kScanBlock, (unsigned long long)((int64_t)dprice * (int32_t)t));
+  red_shared_u64(w + 4 * kScanBlock, (unsigned long long)((int64_t)p * ((100 - (int32_t)d) * (int32_t)t)));
 }
 
 // Block reduction of the per-thread partials into the global 128-bit totals
@@ -76,7 +76,23 @@ __device__ __forceinline__ void block_flush(const unsigned long long* cols, int 
   for (int c = warp; c < n_groups * kWords; c += kScanBlock / 32) {
     const int g = c / kWords, w = c - g * kWords;
     const unsigned long long* col = cols + (size_t)c * kScanBlock + lane;
-    if (w < kWords - 1) {
+    if (!kWide && w < kNarrowPacked) {
+      const int low = narrow_low(w);
+      int64_t s = 0;
+      uint32_t f = 0;
+#pragma unroll
+      for (int i = 0; i < kScanBlock / 32; ++i) {
+        const int64_t v = (int64_t)col[32 * i];
+        s += v >> low;
+        f += (uint32_t)v & ((1u << low) - 1u);
+      }
+      s = warp_sum_i64(s);
+      f = warp_sum_u32(f);
+      if (lane == 0) {
+        raw[g][w] = s;
+        raw[g][kWords + w] = (int64_t)f;
+      }
+    } else if (!kWide || w < kWords - 1) {
       int64_t s = 0;
 #pragma unroll
       for (int i = 0; i < kScanBlock / 32; ++i) s += (int64_t)col[32 * i];
@@ -88,17 +104,12 @@ __device__ __forceinline__ void block_flush(const unsigned long long* cols, int 
       for (int i = 0; i < kScanBlock / 32; ++i) {
         const uint64_t pk = col[32 * i];
         f[0] += (uint32_t)(pk & 0x1ffu);
-        if (kWide) {
-          f[1] += (uint32_t)((pk >> 9) & 0x7fffu);
-          f[2] += (uint32_t)((pk >> 24) & 0x7fffu);
-          f[3] += (uint32_t)(pk >> 39);
-        } else {
-          f[1] += (uint32_t)((pk >> 9) & 0xffffu);
-          f[2] += (uint32_t)(pk >> 25);
-        }
+        f[1] += (uint32_t)((pk >> 9) & 0x7fffu);
+        f[2] += (uint32_t)((pk >> 24) & 0x7fffu);
+        f[3] += (uint32_t)(pk >> 39);
       }
 #pragma unroll
-      for (int j = 0; j < (kWide ? 4 : 3); ++j) {
+      for (int j = 0; j < 4; ++j) {
         const uint32_t s = warp_sum_u32(f[j]);
         if (lane == 0) raw[g][kWords - 1 + j] = (int64_t)s;
       }
@@ -119,16 +130,17 @@ __device__ __forceinline__ void block_flush(const unsigned long long* cols, int 
         case 6: v = r[3]; break;
         default: v = (__int128)r[3] * 100 + r[7]; break;
       }
-    } else {  // 0 price  1 dp  2 dp*(100+t)  3 p*(100-d)  4 p*(100-d)*(100+t)  5 count  6 disc  7 qty + 32768 each
+    } else {  // as narrow_row's words, then the lower fields: 5 qty + 32768 each  6 disc  7 count
+      const __int128 pd = (__int128)r[0] * 100 - r[2];
       switch (i % kQ1Sums) {
-        case 0: v = r[5]; break;
-        case 1: v = r[7] - 32768 * r[5]; break;
+        case 0: v = r[7]; break;
+        case 1: v = r[5] - 32768 * r[7]; break;
         case 2: v = r[0]; break;
         case 3: v = r[6]; break;
         case 4: v = r[1]; break;
-        case 5: v = r[3]; break;
-        case 6: v = r[2]; break;
-        default: v = r[4]; break;
+        case 5: v = pd; break;
+        case 6: v = (__int128)r[1] * 100 + r[3]; break;
+        default: v = pd * 100 + r[4]; break;
       }
     }
     if (v != 0) atomic_add_i128(acc + 2 * i, v);
@@ -240,8 +252,9 @@ __global__ void __launch_bounds__(kScanBlock) q1_lineitem_kernel(bo_lineitem_col
   const int64_t chunks = n >> 3;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  // As in q1_fact_kernel (6.0M rows 32.9 -> 28.7 us).  What bounds it now is the
-  // shared-memory pipe (85 % busy): six words of a row read and written.
+  // As in q1_fact_kernel (6.0M rows 32.9 -> 28.7 us; 26.4 with five words a row
+  // instead of six).  What bounds it is the shared-memory pipe (85 % busy with
+  // six words); three blocks a SM in 80 registers took 31.5 against 29.1 us.
   LineitemChunk cur, nxt;
   if (tid < chunks) cur.load(c, tid << 3);
   for (int64_t ch = tid; ch < chunks; ch += stride) {
