@@ -7,7 +7,7 @@
 //          share of the items, finds every chunk's number of smaller items by
 //          binary search; their sum is the item's rank, and its value goes there.
 //          Lanes search neighbouring chunks, so a chunk takes 257 places: with
-//          256 they met in one bank (16 us instead of 10 for 11K items).
+//          256 they met in one bank (16 us instead of 10 for 11K items and 512 threads).
 // Short chunks, because a block's searches serialise on its SM's shared memory
 // (chunks of 2048 items: 20 us for 11K items on six SMs); searches through L1
 // (8 to 18 us) are bound by one 128-byte line per cycle.
@@ -15,7 +15,7 @@
 // total whatever order the items came in.  A count above the limit sets
 // *overflow and sorts nothing: the caller sorts another way.  Against one
 // thread-block cluster's radix sort (cluster_sort_kernel), whose every 8-bit
-// digit is a round of cluster barriers: 15 us against 32 for Q3's 11K rows, 13
+// digit is a round of cluster barriers: 13 us against 32 for Q3's 11K rows, 10
 // against 43 for Q18's 7K rows (whose two keys are two sorts there).
 #pragma once
 
@@ -30,7 +30,7 @@ constexpr int kSsChunk = 256;
 constexpr int kSsRow = kSsChunk + 1;      // places of a chunk in shared memory
 constexpr int64_t kSmallSortMax = 24576;  // their keys: 193 KB of shared memory
 constexpr int kSsChunks = (int)(kSmallSortMax / kSsChunk);
-constexpr int kSsRankBlock = 512;
+constexpr int kSsRankBlock = 768;  // 512: Q3 71 us instead of 68, Q18 75 instead of 70; 1024 the same
 constexpr size_t kSsSmem = (size_t)kSsChunks * kSsRow * sizeof(unsigned long long);
 
 // The sorted chunks: keys apart from {tie, value}, which are read once per item
