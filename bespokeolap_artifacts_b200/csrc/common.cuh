@@ -39,6 +39,32 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 // ---------------------------------------------------------------- loads ----
+// What a kernel launched dependently reads of its predecessors' output, after
+// pdl_wait(): coherent loads, which stay behind the wait.  (A read-only load,
+// __ldg or one through a const __restrict__ pointer, may be moved before it: such
+// data is not constant for the kernel's lifetime.)
+template <typename T>
+__device__ __forceinline__ T ld_prior(const T* p) {
+  static_assert(sizeof(T) == 1 || sizeof(T) == 4 || sizeof(T) == 8, "one register or two");
+  if constexpr (sizeof(T) == 1) {
+    uint32_t v;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+    return (T)v;
+  } else if constexpr (sizeof(T) == 4) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return (T)v;
+  } else {
+    unsigned long long v;
+    asm volatile("ld.global.u64 %0, [%1];" : "=l"(v) : "l"(p));
+    return (T)v;
+  }
+}
+__device__ __forceinline__ uint4 ld_prior_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
 // Streaming 128-bit loads: read-only, not allocated in L1 (each byte of a fact
 // column is touched exactly once per scan).
 __device__ __forceinline__ int4 ld_stream_v4(const void* p) {
@@ -80,6 +106,15 @@ __device__ __forceinline__ int8v ld_stream_v8(const void* p) {
 __device__ __forceinline__ int8v ld_first_v8(const void* p) {
   int8v r;
   asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.s32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+                 "=r"(r.v[6]), "=r"(r.v[7])
+               : "l"(p));
+  return r;
+}
+// ld_first_v8 of a predecessor's output.
+__device__ __forceinline__ int8v ld_prior_v8(const void* p) {
+  int8v r;
+  asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.s32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
                  "=r"(r.v[6]), "=r"(r.v[7])
                : "l"(p));

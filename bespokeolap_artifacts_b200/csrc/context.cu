@@ -84,8 +84,8 @@ __global__ void __launch_bounds__(256) result_kernel(const uint32_t* __restrict_
                                                      const uint32_t* __restrict__ err, uint32_t* host,
                                                      uint32_t* host_err) {
   pdl_wait();
-  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) host[i] = record[i];
-  if (threadIdx.x == 0) *host_err = *err;
+  for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) host[i] = ld_prior(record + i);
+  if (threadIdx.x == 0) *host_err = ld_prior(err);
 }
 }  // namespace
 

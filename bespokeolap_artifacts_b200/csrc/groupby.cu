@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(256) gd_cfilter_kernel(bo_gb_c_cols c, CatSet 
 
 // Whether the filtered scan runs.
 __device__ __forceinline__ bool gd_filtered(const GbMeta* meta, bool has_filter) {
-  return has_filter && !__ldcg(&meta->no_filter) && __ldcg(&meta->c_pass) <= kGdFilterKeys;
+  return has_filter && !ld_prior(&meta->no_filter) && ld_prior(&meta->c_pass) <= kGdFilterKeys;
 }
 
 // A block's pre-aggregation of heavy hitters, as gb_scan_kernel's, which a warp
@@ -982,7 +982,7 @@ __global__ void __launch_bounds__(kGdBlock, 1) gd_scan_kernel(bo_gb_b_cols b, in
         const uint32_t i = i0 + r * 32 + lane;
         c[r] = i < qn ? qc[i] : 0xffffffffu;
         row[r] = i < qn ? qr[i] : 0u;
-        y[r] = c[r] < nc ? __ldg(code + c[r]) : 0u;
+        y[r] = c[r] < nc ? ld_prior(code + c[r]) : 0u;
       }
 #pragma unroll
       for (int r = 0; r < kGdResolveR; ++r) a[r] = y[r] ? __ldg(b.a_id + row[r]) : -1;
@@ -1069,11 +1069,11 @@ __global__ void __launch_bounds__(kGpBlock, 1)
     uint4 v = make_uint4(0, 0, 0, 0);
     const uint32_t* src = cbits + lo / 32 + 4 * i;
     if (4 * i + 4 <= words) {
-      v = __ldcg(reinterpret_cast<const uint4*>(src));
+      v = ld_prior_v4(src);
     } else {
-      if (4 * i < words) v.x = __ldcg(src);
-      if (4 * i + 1 < words) v.y = __ldcg(src + 1);
-      if (4 * i + 2 < words) v.z = __ldcg(src + 2);
+      if (4 * i < words) v.x = ld_prior(src);
+      if (4 * i + 1 < words) v.y = ld_prior(src + 1);
+      if (4 * i + 2 < words) v.z = ld_prior(src + 2);
     }
     reinterpret_cast<uint4*>(gp_bits)[i] = v;
   }
@@ -1131,7 +1131,7 @@ __global__ void __launch_bounds__(kGaBlock, 8)
       uint32_t plane[kGpMaxRanges];  // requested together
 #pragma unroll
       for (uint32_t r = 0; r < (uint32_t)kGpMaxRanges; ++r)
-        plane[r] = r < ranges ? __ldg(planes + r * plane_bytes + st * 32 + (threadIdx.x & 31)) : 0u;
+        plane[r] = r < ranges ? ld_prior(planes + r * plane_bytes + st * 32 + (threadIdx.x & 31)) : 0u;
 #pragma unroll
       for (int r = 0; r < kGpMaxRanges; ++r) hit |= plane[r];
     } else {
@@ -1152,8 +1152,8 @@ __global__ void __launch_bounds__(kGaBlock, 8)
         continue;
       }
       const bool in = in_a && (uint32_t)cid[k] < nc;
-      if (kYear) y[k] = in ? __ldg(code + cid[k]) : 0u;
-      else y[k] = in ? (__ldg(cbits + (cid[k] >> 5)) >> (cid[k] & 31)) & 1u : 0u;
+      if (kYear) y[k] = in ? ld_prior(code + cid[k]) : 0u;
+      else y[k] = in ? (ld_prior(cbits + (cid[k] >> 5)) >> (cid[k] & 31)) & 1u : 0u;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -1261,14 +1261,14 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
     const int64_t id0 = t * kGcTile + threadIdx.x * kGcPer;
     if (id0 + kGcPer <= n_ids) {
       if (kPairs) {
-        const int8v v0 = ld_first_v8(entries + 2 * id0), v1 = ld_first_v8(entries + 2 * id0 + 8);
+        const int8v v0 = ld_prior_v8(entries + 2 * id0), v1 = ld_prior_v8(entries + 2 * id0 + 8);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           c[j] = (uint32_t)v0.v[2 * j];
           c[4 + j] = (uint32_t)v1.v[2 * j];
         }
       } else {
-        const int8v v = ld_first_v8(entries + id0);
+        const int8v v = ld_prior_v8(entries + id0);
 #pragma unroll
         for (int j = 0; j < 8; ++j) c[j] = (uint32_t)v.v[j];
       }
@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
       for (int j = 0; j < kGcPer; ++j) {
         const int64_t id = id0 + j;
         c[j] = 0;
-        if (id < n_ids && ((__ldg(amask + (id >> 5)) >> (id & 31)) & 1u)) c[j] = entries[kPairs ? 2 * id : id];
+        if (id < n_ids && ((__ldg(amask + (id >> 5)) >> (id & 31)) & 1u)) c[j] = ld_prior(entries + (kPairs ? 2 * id : id));
       }
     }
   };
@@ -1408,7 +1408,7 @@ __global__ void __launch_bounds__(kGcBlock, 3) gd_collect_kernel(const uint32_t*
     const uint32_t id = (uint32_t)(key & ((1ull << wa) - 1ull));
     bo_gb_row r;
     r.a_id = (int32_t)id;
-    r.min_year = kPairs ? year_lo + (int32_t)(kGdYearTop - entries[2 * (size_t)id + 1]) - 1 : 0x7fffffff;
+    r.min_year = kPairs ? year_lo + (int32_t)(kGdYearTop - ld_prior(entries + 2 * (size_t)id + 1)) - 1 : 0x7fffffff;
     r.count = (int64_t)(cmax - (key >> wa));
     out->rows[threadIdx.x] = r;
   }
@@ -1467,7 +1467,7 @@ __global__ void __launch_bounds__(256) gd_years_kernel(bo_gb_b_cols b, int64_t n
       for (int i = 0; i < rows; ++i) {
         if (key[i] != a[j]) continue;
         const int32_t c = b.c_id[r];
-        const uint32_t y = (uint32_t)c < (uint32_t)n_c ? __ldg(code + c) : 0u;
+        const uint32_t y = (uint32_t)c < (uint32_t)n_c ? ld_prior(code + c) : 0u;
         if (y) atomicMin(&out->rows[i].min_year, year_lo + (int32_t)y - 1);
       }
     }

@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(kBuildBlock) join_build_kernel(bo_join_build_c
       waited = true;
       // Read-only for this kernel (written by the init kernel): the L1-cached
       // path avoids every warp hitting the same L2 sector.
-      mask = (1ull << __ldg(&meta->cap_log2)) - 1;
-      n_bits = __ldg(&meta->n_bits);
+      mask = (1ull << ld_prior(&meta->cap_log2)) - 1;
+      n_bits = ld_prior(&meta->n_bits);
     }
     qual += __popc(q);
     // Compact the qualifying keys of the whole warp into its queue so the CAS
@@ -375,7 +375,7 @@ __device__ __forceinline__ void probe_emit(const int32_t* qf, const uint16_t* qo
       key[r] = ok ? qf[i] : 0;
       row[r] = ok ? base + qo[i] : 0;
       idx[r] = hash32((uint32_t)key[r]) & mask;
-      v[r] = ok ? __ldg(slots + idx[r]) : kEmptySlot;
+      v[r] = ok ? ld_prior(slots + idx[r]) : kEmptySlot;
     }
     unsigned long long mult[R];
     uint32_t bal[R], n = 0;
@@ -432,14 +432,14 @@ static __device__ __noinline__ ProbeAcc probe_bits(const bo_join_probe_cols p, c
 #pragma unroll
     for (int j = 0; j < kRows; ++j) {
       const bool ok = r + 32 * j < n && key[j] < n_bits;
-      hit |= (ok ? (__ldg(bits + (key[j] >> 5)) >> (key[j] & 31u)) & 1u : 0u) << j;
+      hit |= (ok ? (ld_prior(bits + (key[j] >> 5)) >> (key[j] & 31u)) & 1u : 0u) << j;
     }
     unsigned long long mult[kRows];
     if constexpr (kHashed) {
       unsigned long long v[kRows];
 #pragma unroll
       for (int j = 0; j < kRows; ++j)
-        v[j] = r + 32 * j < n && bloom_test(bl, wmask, key[j]) ? __ldg(slots + (hash32(key[j]) & mask)) : kEmptySlot;
+        v[j] = r + 32 * j < n && bloom_test(bl, wmask, key[j]) ? ld_prior(slots + (hash32(key[j]) & mask)) : kEmptySlot;
 #pragma unroll
       for (int j = 0; j < kRows; ++j) {
         mult[j] = (hit >> j) & 1u;
@@ -488,7 +488,7 @@ __device__ __forceinline__ bool probe_finish(const ProbeAcc& acc, unsigned __int
     res.match_count = narrow_i64(m, fbad);
     res.sum_trunc = to_bo_i128(t);
     res.sum_exact = to_bo_i128(t * 100 + rr);
-    res.capacity_log2 = __ldg(&meta->cap_log2);
+    res.capacity_log2 = ld_prior(&meta->cap_log2);
     res.overflowed = (int32_t)__ldcg(&meta->overflow);
     res.reruns = 0;
     res.mode = mode;
@@ -585,11 +585,11 @@ __global__ void __launch_bounds__(kJoinBlock, 2) join_probe_kernel(bo_join_probe
   __syncthreads();
   const uint32_t* bl = use_bloom ? bloom_s : &all_ones;
   const uint32_t wmask = use_bloom ? (kBloomWords - 1u) : 0u;
-  const uint64_t mask = (1ull << __ldg(&meta->cap_log2)) - 1;
-  const uint32_t n_bits = kBits ? __ldg(&meta->n_bits) : 0u;
+  const uint64_t mask = (1ull << ld_prior(&meta->cap_log2)) - 1;
+  const uint32_t n_bits = kBits ? ld_prior(&meta->n_bits) : 0u;
   if (n_bits) {
     const uint32_t bad = acc.bad;
-    acc = __ldg(&meta->hashed) ? probe_bits<true>(p, bits, n_bits, slots, mask, probe_limit, bl, wmask)
+    acc = ld_prior(&meta->hashed) ? probe_bits<true>(p, bits, n_bits, slots, mask, probe_limit, bl, wmask)
                                : probe_bits<false>(p, bits, n_bits, slots, mask, probe_limit, bl, wmask);
     acc.bad |= bad;
   } else {
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(kSmemBlock, 1) join_probe_smem_kernel(bo_join_
   load(st, f1);
   load(st + nwarps, f2);
   pdl_wait();  // launched behind the build kernel
-  const bool hashed = __ldg(&meta->hashed) != 0;
+  const bool hashed = ld_prior(&meta->hashed) != 0;
   if (threadIdx.x == 0) {
     const uint32_t bytes = hashed ? kBloomBytes : n_bits / 8;
     mbar_init(&bar, 1);
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(kSmemBlock, 1) join_probe_smem_kernel(bo_join_
   if (!copied) acc.bad |= kErrSpinTimeout;
   __syncthreads();
   if (hashed) {
-    const uint64_t mask = (1ull << __ldg(&meta->cap_log2)) - 1;
+    const uint64_t mask = (1ull << ld_prior(&meta->cap_log2)) - 1;
     int32_t* qf = reinterpret_cast<int32_t*>(smem + kBloomWords) + warp * kQueue;
     uint16_t* qo = reinterpret_cast<uint16_t*>(smem + kBloomWords + kSmemWarps * kQueue) + warp * kQueue;
     probe_hashed<false>(p, slots, mask, probe_limit, copied ? smem : &all_ones, copied ? kBloomWords - 1u : 0u, qf, qo,

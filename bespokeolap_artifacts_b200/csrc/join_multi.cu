@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_count_kernel(bo_join_build_c
   __shared__ uint32_t h[(kMq + 1) * kMqClassCopies];
   pdl_launch_dependents();
   pdl_wait();
-  if (__ldcg(&st->dense)) return;
+  if (ld_prior(&st->dense)) return;
   mq_load_queries(q, qv);
   for (int i = threadIdx.x; i < (kMq + 1) * kMqClassCopies; i += kMqBuildBlock) h[i] = 0;
   __syncthreads();
@@ -277,12 +277,12 @@ __global__ void mq_init_kernel(unsigned long long* slots, uint32_t* bloom, MqSta
   pdl_wait();
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (__ldg(&st->dense)) {
+  if (ld_prior(&st->dense)) {
     uint4* v = reinterpret_cast<uint4*>(slots);
-    for (uint64_t i = tid; i < ((uint64_t)__ldg(&st->range) + 15) / 16; i += stride) v[i] = make_uint4(0, 0, 0, 0);
+    for (uint64_t i = tid; i < ((uint64_t)ld_prior(&st->range) + 15) / 16; i += stride) v[i] = make_uint4(0, 0, 0, 0);
     return;
   }
-  const int32_t cl = __ldg(&st->cap_log2);
+  const int32_t cl = ld_prior(&st->cap_log2);
   const uint64_t cap = 1ull << cl;
   ulonglong2* s2 = reinterpret_cast<ulonglong2*>(slots);
   for (uint64_t i = tid; i < cap / 2; i += stride) s2[i] = make_ulonglong2(kEmptySlot, kEmptySlot);
@@ -302,10 +302,10 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_build_dense_kernel(bo_join_b
   mq_load_queries(q, qv);
   for (int i = threadIdx.x; i < (kMq + 1) * kMqClassCopies; i += kMqBuildBlock) h[i] = 0;
   pdl_wait();
-  if (!__ldg(&st->dense)) return;
+  if (!ld_prior(&st->dense)) return;
   __syncthreads();
   const uint32_t copy = threadIdx.x & (kMqClassCopies - 1);
-  const uint32_t base = __ldg(&st->base);
+  const uint32_t base = ld_prior(&st->base);
   const int64_t chunks = (b.n_rows + kMqBuildRows - 1) / kMqBuildRows;
   uint32_t dup = 0;
   for (int64_t c = (int64_t)blockIdx.x * kMqBuildBlock + threadIdx.x; c < chunks;
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_build_dense_kernel(bo_join_b
     for (int j = 0; j < kMqBuildRows; ++j) dup |= (old[j] >> (8 * ((key[j] - base) & 3u))) & 0xffu;
   }
   if (__any_sync(0xffffffffu, dup != 0) && (threadIdx.x & 31) == 0) atomicOr(&st->dup, 1u);
-  if (!__ldg(&st->counted)) mq_count_finish(h, q, st, max_log2);
+  if (!ld_prior(&st->counted)) mq_count_finish(h, q, st, max_log2);
 }
 
 __device__ __forceinline__ void mq_insert(unsigned long long* slots, uint32_t* bloom, uint64_t mask, int32_t key,
@@ -354,12 +354,12 @@ __global__ void __launch_bounds__(kMqBuildBlock) mq_build_kernel(bo_join_build_c
                                                                  MqState* st) {
   pdl_launch_dependents();
   pdl_wait();
-  if (__ldg(&st->dense)) return;
+  if (ld_prior(&st->dense)) return;
   __shared__ MultiQ q;
   __shared__ uint32_t queue[kMqBuildBlock / 32][2][32 * kMqBuildRows];
   mq_load_queries(q, qv);
   __syncthreads();
-  const uint64_t mask = (1ull << __ldcg(&st->cap_log2)) - 1;
+  const uint64_t mask = (1ull << ld_prior(&st->cap_log2)) - 1;
   const int lane = threadIdx.x & 31;
   uint32_t* qk = queue[threadIdx.x >> 5][0];
   uint32_t* qm = queue[threadIdx.x >> 5][1];
@@ -501,12 +501,12 @@ __global__ void __launch_bounds__(kMqDenseBlock) mq_probe_dense_kernel(bo_join_p
                                                                        bo_join_result* out, MultiQ qv, uint32_t* err) {
   pdl_launch_dependents();
   pdl_wait();
-  if (!__ldg(&st->dense)) return;
+  if (!ld_prior(&st->dense)) return;
   constexpr int kWarps = kMqDenseBlock / 32;
   __shared__ __align__(16) MqWarpAcc wa[kWarps];
   for (int i = threadIdx.x; i < (int)(sizeof(wa) / 4); i += kMqDenseBlock) reinterpret_cast<uint32_t*>(wa)[i] = 0;
   __syncthreads();
-  const uint32_t base_key = __ldg(&st->base), range = __ldg(&st->range);
+  const uint32_t base_key = ld_prior(&st->base), range = ld_prior(&st->range);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n = p.n_rows;
   constexpr int kStep = 32 * kMqRowsPerLane;
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(kMqDenseBlock) mq_probe_dense_kernel(bo_join_p
     for (int j = 0; j < kMqRowsPerLane; ++j)
       off[j] = r0 + 32 * j < n ? (uint32_t)__ldcs(p.fk + r0 + 32 * j) - base_key : ~0u;
 #pragma unroll
-    for (int j = 0; j < kMqRowsPerLane; ++j) code[j] = off[j] < range ? __ldg(bytes + off[j]) : 0u;
+    for (int j = 0; j < kMqRowsPerLane; ++j) code[j] = off[j] < range ? ld_prior(bytes + off[j]) : 0u;
     uint64_t pr[kMqRowsPerLane], dc[kMqRowsPerLane];
 #pragma unroll
     for (int j = 0; j < kMqRowsPerLane; ++j) {
@@ -558,7 +558,7 @@ __device__ __forceinline__ void mq_resolve(const int32_t* qf, const uint8_t* qo,
       key[r] = ok ? qf[i] : 0;
       row[r] = ok ? base + qo[i] : 0;
       idx[r] = hash32((uint32_t)key[r]) & mask;
-      v[r] = ok ? __ldg(slots + idx[r]) : kEmptySlot;
+      v[r] = ok ? ld_prior(slots + idx[r]) : kEmptySlot;
     }
     uint32_t code[R];
 #pragma unroll
@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_col
                                                               bo_join_result* out, MultiQ qv, uint32_t* err) {
   pdl_launch_dependents();
   pdl_wait();
-  if (__ldg(&st->dense)) return;
+  if (ld_prior(&st->dense)) return;
   extern __shared__ __align__(128) uint32_t bloom_s[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int32_t q_fk[kMqWarps][32 * kMqRowsPerLane];
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(kMqBlock, 2) mq_probe_kernel(bo_join_probe_col
   const uint32_t wmask = use_bloom ? (kBloomWords - 1u) : 0u;
   MqAcc acc;
   if (!use_bloom) acc.bad |= kErrSpinTimeout;
-  const uint64_t mask = (1ull << __ldcg(&st->cap_log2)) - 1;
+  const uint64_t mask = (1ull << ld_prior(&st->cap_log2)) - 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int32_t* qf = q_fk[warp];
   uint8_t* qo = q_off[warp];

@@ -201,7 +201,7 @@ static __device__ __noinline__ unsigned long long probe_slow(const unsigned long
   const uint64_t steps = mask < limit ? mask : limit;
   for (uint64_t step = 1; step <= steps; ++step) {
     idx = (idx + 1) & mask;
-    const unsigned long long v = kCoherent ? __ldcg(slots + idx) : __ldg(slots + idx);
+    const unsigned long long v = kCoherent ? __ldcg(slots + idx) : ld_prior(slots + idx);
     if (v == kEmptySlot) return 0;
     if ((uint32_t)(v >> 32) == key) return v & 0xffffffffull;
   }
@@ -231,7 +231,7 @@ __device__ __forceinline__ void probe_resolve(const int32_t* qf, const uint16_t*
       key[r] = ok ? qf[i] : 0;
       row[r] = ok ? base + qo[i] : 0;
       idx[r] = hash32((uint32_t)key[r]) & mask;
-      v[r] = ok ? (kCoherent ? __ldcg(slots + idx[r]) : __ldg(slots + idx[r])) : kEmptySlot;
+      v[r] = ok ? (kCoherent ? __ldcg(slots + idx[r]) : ld_prior(slots + idx[r])) : kEmptySlot;
     }
     unsigned long long mult[R];
 #pragma unroll

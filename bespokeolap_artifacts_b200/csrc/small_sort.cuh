@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(kSsChunk) ss_chunk_kernel(Make make, const uns
   __shared__ uint4 buf[2][kSsChunk];
   pdl_launch_dependents();
   pdl_wait();
-  const unsigned long long n = *n_dev;
+  const unsigned long long n = ld_prior(n_dev);
   if (n > (unsigned long long)kSmallSortMax) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *overflow = 1u;
     return;
@@ -109,14 +109,14 @@ static __global__ void __launch_bounds__(kSsRankBlock) ss_rank_kernel(SsItems it
   __shared__ uint32_t rank[kSsRankBlock];
   pdl_launch_dependents();
   pdl_wait();
-  const unsigned long long nd = *n_dev;
+  const unsigned long long nd = ld_prior(n_dev);
   if (nd > (unsigned long long)kSmallSortMax) return;
   const uint32_t n = (uint32_t)nd, chunks = (n + kSsChunk - 1) / kSsChunk;
   const uint32_t share = (n + gridDim.x - 1) / gridDim.x;  // <= kSsRankBlock (the host's grid)
   const uint32_t e0 = blockIdx.x * share, mine = e0 >= n ? 0u : (n - e0 < share ? n - e0 : share);
   if (mine == 0) return;
   for (uint32_t i = threadIdx.x; i < chunks * kSsChunk; i += kSsRankBlock)
-    ss_keys[i / kSsChunk * kSsRow + i % kSsChunk] = __ldg(items.key + i);
+    ss_keys[i / kSsChunk * kSsRow + i % kSsChunk] = ld_prior(items.key + i);
   rank[threadIdx.x] = 0;
   __syncthreads();
   for (uint32_t w = threadIdx.x; w < mine * chunks; w += kSsRankBlock) {
@@ -129,7 +129,7 @@ static __global__ void __launch_bounds__(kSsRankBlock) ss_rank_kernel(SsItems it
       const unsigned long long* run = ss_keys + c * kSsRow;
       auto before = [&](uint32_t j) {  // the chunk's item j before item i
         const unsigned long long k = run[j];
-        return k < key || (k == key && __ldg(&items.rest[c * kSsChunk + j].x) < __ldg(&items.rest[i].x));
+        return k < key || (k == key && ld_prior(&items.rest[c * kSsChunk + j].x) < ld_prior(&items.rest[i].x));
       };
 #pragma unroll
       for (uint32_t half = kSsChunk / 2; half > 0; half >>= 1)
@@ -139,7 +139,7 @@ static __global__ void __launch_bounds__(kSsRankBlock) ss_rank_kernel(SsItems it
     atomicAdd(rank + e, at);
   }
   __syncthreads();
-  if (threadIdx.x < mine) out_vals[rank[threadIdx.x]] = items.rest[e0 + threadIdx.x].y;
+  if (threadIdx.x < mine) out_vals[rank[threadIdx.x]] = ld_prior(&items.rest[e0 + threadIdx.x].y);
 }
 
 // Sorts the *n_dev items make(0) .. make(n - 1) and writes their values in

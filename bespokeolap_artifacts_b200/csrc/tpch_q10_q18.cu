@@ -343,13 +343,13 @@ __global__ void __launch_bounds__(kTpBlock) q18_qualify_kernel(const int32_t* __
         if (in) ok |= 1u << j;
         else raise_error(err, kErrValueRange);
       }
-      qty[j] = in ? __ldg(sum + key[j]) : 0;
+      qty[j] = in ? ld_prior(sum + key[j]) : 0;
     }
 #pragma unroll
     for (int j = 0; j < kQ18Orders; ++j) {
       const int64_t row = b0 + j * kTpBlock + threadIdx.x;
       if (!((ok >> j) & 1u) || qty[j] <= threshold) continue;
-      if (mark && !((mark[key[j] >> 5] >> (key[j] & 31)) & 1u)) continue;
+      if (mark && !((ld_prior(mark + (key[j] >> 5)) >> (key[j] & 31)) & 1u)) continue;
       if (cust.row_of(o_custkey[row]) < 0) continue;
       mine[atomicAdd(&n_mine, 1u)] = make_uint2((uint32_t)key[j] ^ 0x80000000u, (uint32_t)row);
     }
@@ -413,11 +413,11 @@ __global__ void __launch_bounds__(kQ18RowsBlock) q18_gather_kernel(
        base += (unsigned long long)gridDim.x * kQ18RowsBlock) {
     const unsigned long long i = base + threadIdx.x;
     if (i < n) {
-      const uint32_t row = vals[i];
+      const uint32_t row = ld_prior(vals + i);
       const int32_t key = dense ? (int32_t)(row + 1) : o_orderkey[row];
       const int32_t c = o_custkey[row];
       bo_tpch_q18_row r;
-      r.sum_qty_raw = (int64_t)sum[key];
+      r.sum_qty_raw = (int64_t)ld_prior(sum + key);
       r.custkey = c;
       r.cust_row = cust.row_of(c);
       r.orderkey = key;

@@ -70,7 +70,7 @@ __global__ void q3_orders_kernel(const int32_t* __restrict__ o_orderkey, const i
     }
 #pragma unroll
     for (int j = 0; j < kRows; ++j)
-      take |= (uint32_t)(c[j] >= 0 && c[j] < bound && ((mask[c[j] >> 5] >> (c[j] & 31)) & 1u)) << j;
+      take |= (uint32_t)(c[j] >= 0 && c[j] < bound && ((ld_prior(mask + (c[j] >> 5)) >> (c[j] & 31)) & 1u)) << j;
     if (!take) continue;
 #pragma unroll
     for (int j = 0; j < kRows; ++j) key[j] = (take >> j) & 1u ? o_orderkey[i0 + j * stride] : -1;
@@ -176,9 +176,9 @@ __global__ void __launch_bounds__(kQ3RowsBlock) q3_gather_kernel(
   for (int64_t base = (int64_t)blockIdx.x * kQ3RowsBlock; base < n; base += (int64_t)gridDim.x * kQ3RowsBlock) {
     const int64_t i = base + threadIdx.x;
     if (i < n) {
-      const uint32_t row = vals[i];
+      const uint32_t row = ld_prior(vals + i);
       bo_tpch_q3_row r;
-      r.revenue_raw = (int64_t)rev[row];
+      r.revenue_raw = (int64_t)ld_prior(rev + row);
       r.orderkey = o_orderkey[row];
       r.shippriority = o_shippriority ? o_shippriority[row] : 0;
       r.orderdate_offset = o_orderdate[row];
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kQ3Block) q3_lineitem_kernel(const int32_t* __
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int16_t d = (int16_t)((sw[k >> 1] >> (16 * (k & 1))) & 0xffffu);
-      word[k] = d > date_offset && key[k] >= 0 && (int64_t)key[k] < n_map ? __ldg(qual + (key[k] >> 5)) : 0u;
+      word[k] = d > date_offset && key[k] >= 0 && (int64_t)key[k] < n_map ? ld_prior(qual + (key[k] >> 5)) : 0u;
     }
 #pragma unroll
     for (int k = 0; k < 8; ++k)
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kQ3Block) q3_lineitem_kernel(const int32_t* __
   for (int64_t i = (chunks << 3) + tid; i < n; i += stride) {
     if (l_shipdate[i] <= date_offset) continue;
     const int32_t key = l_orderkey[i];
-    if (key < 0 || (int64_t)key >= n_map || !((__ldg(qual + (key >> 5)) >> (key & 31)) & 1u)) continue;
+    if (key < 0 || (int64_t)key >= n_map || !((ld_prior(qual + (key >> 5)) >> (key & 31)) & 1u)) continue;
     qualifies(i, key);
   }
   __syncthreads();

@@ -212,7 +212,8 @@ int bo_q6_lineitem_host(bo_ctx* ctx, const bo_lineitem_cols* host_cols, int16_t 
  * (builder_impl.cpp:930-991); here the qualifying build keys go into an
  * open-addressing table in HBM (64-bit slots key<<32 | multiplicity, inserted
  * with atomicCAS) plus a blocked Bloom filter the probe stages into shared
- * memory.  Inner-join semantics: a probe row contributes once per matching
+ * memory; device-column forms keep keys as single bits where that is cheaper
+ * (16 bits per build row of scratch).  Inner-join semantics: a probe row contributes once per matching
  * build row. */
 typedef struct bo_join_build_cols {
   const int32_t* key;
@@ -281,7 +282,9 @@ int bo_join_host(bo_ctx* ctx, const bo_join_build_cols* build_host, const bo_joi
  * rows that pass a global Bloom filter of them are split by the top bits of
  * their key's hash (record arrays sized by the row counts, counting scatter),
  * then one block per partition joins the partition in a shared-memory table
- * (8192 slots), so no lookup leaves the SM.  The caller picks the fan-out
+ * (8192 slots), so no lookup leaves the SM.  Calls of 4M rows and more (both
+ * sides) keep one bit per 32-bit key in a 512 MB table instead where that can be
+ * had, with the same results, overflow included.  The caller picks the fan-out
  * (learned.JoinSizer.fanout on the predicted qualifying rows: a single pass
  * while its table stays in L2, else partitions of about 4096 keys).  A
  * partition with more distinct keys than its table holds sets overflowed;
@@ -294,8 +297,8 @@ int bo_join_partitioned(bo_ctx* ctx, const bo_join_build_cols* build, const bo_j
 
 /* Shared joins: n_queries (1..BO_JOIN_MULTI_MAX) filtered joins of the same
  * build and probe tables that differ only in their predicate constants, in
- * one count, one build and one probe pass (the table maps a key to the mask
- * of the queries it qualifies for).  out[i] is the result bo_join_plain
+ * one build and one probe pass (the table maps a key to its class: the first
+ * of its segment's queries, in date_lt order, that it qualifies for).  out[i] is the result bo_join_plain
  * returns for params[i] (capacity_log2 is the shared table's).  No reference
  * counterpart: it serves concurrent requests (the reference runs one query
  * per call, bespoke_tpch/query_impl.cpp:159-388).  A key that qualifies
@@ -419,7 +422,9 @@ int bo_groupby_topk_presized(bo_ctx* ctx, const bo_gb_a_cols* a, const bo_gb_b_c
  * survivor makes at most one) while that stays within 16 GiB, else they are
  * sized from predicted_joined_rows.  A record buffer or partition table that
  * turns out too small sets overflowed; bo_groupby_topk_partitioned then
- * reruns the plain form. */
+ * reruns the plain form.  Where one entry per a_id fits the group table's
+ * memory and the years a byte, entries are indexed by a_id instead, with the
+ * same results, overflow included. */
 #define BO_GB_MAX_LOG2_PARTITIONS 14
 int bo_groupby_topk_partitioned_device(bo_ctx* ctx, const bo_gb_a_cols* a, const bo_gb_b_cols* b,
                                        const bo_gb_c_cols* c, const bo_gb_params* params, int32_t log2_partitions,
