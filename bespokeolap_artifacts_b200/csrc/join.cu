@@ -66,7 +66,7 @@ constexpr int64_t kBitsPerRow = 16;
 // beside its queues).  They answer every row, so matches need no look at the
 // table; a key without a bit, or a repeated one, leaves the probe to the filter
 // and the table.  Filter against bits: 250 thousand x 1M rows 26.6 / 23.5 us, 1.5M
-// x 6M with 60 / 120 / 300 thousand keys 39 / 35, 50 / 41 and 77 / 57 us.
+// x 6M with 60 / 120 / 300 thousand keys 39 / 34, 50 / 41 and 77 / 57 us.
 constexpr int64_t kSmemBits = 1536000;
 
 // Device-resident join state (one per context, in the "join_meta" region).
@@ -613,9 +613,13 @@ __global__ void __launch_bounds__(kJoinBlock, 2) join_probe_kernel(bo_join_probe
 // warp requests its first two steps' fk before it waits for the build, and
 // each further step two steps ahead; its matches queue up across steps until
 // 64 of them load their price and discount together.  Bound by latency at 6M
-// rows (five steps a warp): the copy of the bits, the payload's round trips and
+// rows (seven steps a warp): the copy of the bits, the payload's round trips and
 // the block totals; 70 MB of DRAM reads, sparse payload among them, are 11 us.
-constexpr int kSmemBlock = 1024;
+// 768 threads leave a SM the registers and the memory of one build block, so that
+// the probe starts beside the build, or another query's build beside it: 35.5 us
+// a query of 1.5M x 6M rows, 33.3 with two in flight, against 36.7 and 34.6 with
+// 1024 threads (and 38.5 and 33.5 with the filter).
+constexpr int kSmemBlock = 768;
 constexpr int kSmemWarps = kSmemBlock / 32;
 constexpr uint32_t kSmemFlushAt = 64;
 constexpr int kSmemQueue = (int)kSmemFlushAt + kRowsPerWarpStep;  // matches per warp: (step, row of the step)
